@@ -12,7 +12,7 @@
 // parallel-transport convolutions of Lehner & Wettig, "Gauge-equivariant
 // neural networks as preconditioners in lattice QCD", PRD 108 (2023).
 //
-// Forward kernel, one CTA per tile of 42 sites = 126 rows (site, colour):
+// Forward kernel, tiles of 32 sites = 96 rows (site, colour):
 //  1. the CUDA cores transport every input channel along the 9 displacements
 //     and write the real GEMM operand A[row][k], k = (2d + re/im)*C_in + i,
 //     in BF16 into shared memory in the canonical K-major no-swizzle UMMA
@@ -20,16 +20,19 @@
 //  2. one thread issues tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M=128)
 //     against the packed real weight matrix B[n][k] (n = 2*o + re/im), the
 //     accumulator lives in tensor memory;
-//  3. the four warps read their 32 accumulator lanes back (tcgen05.ld) and
+//  3. three warps read their 32 accumulator lanes back (tcgen05.ld) and
 //     store the output channels in FP32.
 // Every wait on the MMA's mbarrier is bounded: on time-out the kernel sets
 // an error flag, skips the read-back, frees its tensor memory and returns.
 //
-// Backward: dA = dY B (tcgen05, same machinery), then the adjoint transport
-// (a gather) gives d in; dB = A^T dY per tile on the CUDA cores with a
-// deterministic reduction over tiles.
+// Backward: the gradient of the input is a layer of the same kind on dY, with
+// adjoint weights and the displacements reversed (T_{+mu}^dag = T_{-mu}), so it
+// runs in the forward kernels; dB = A^T dY accumulates in registers over a
+// CTA's tiles on the tensor cores (mma.sync, the FP32 dY split into three
+// BF16 terms), with a deterministic reduction over the CTAs.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -148,9 +151,6 @@ __host__ __device__ __forceinline__ uint32_t canon(int r, int k, int K) {
   return uint32_t((r >> 3) * (K / 8) * 128 + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
 }
 
-constexpr int kTileSites = 42;  // 126 of the 128 MMA rows
-constexpr int kThreads = 128;
-
 template <int CIN, int COUT>
 struct Ptc {
   static constexpr int KF = 18 * CIN;
@@ -158,7 +158,6 @@ struct Ptc {
   static constexpr int NF = 2 * COUT;
   static constexpr int NP = NF < 16 ? 16 : (NF + 15) / 16 * 16;
   static constexpr int TCOLS = NP <= 32 ? 32 : 64;
-  static constexpr int A_BYTES = 128 * KP * 2;
   static constexpr int B_BYTES = NP * KP * 2;
   // forward kernel: A holds the 96 rows of 32 sites; the MMA's rows 96..127
   // read the bytes that follow (the weights, padded to at least 32 rows),
@@ -193,77 +192,6 @@ struct PtcGeo {
   int* err;
   const int* skip;  // forward only: when set and nonzero the launch does nothing
 };
-
-// Builds the BF16 A tile: rows (site, colour) of the tile, columns
-// (2d + part)*CIN + i; padding rows/columns are zero.
-template <int CIN, int KP>
-__device__ void build_a_tile(const PtcGeo& G, const float2* __restrict__ in, int site0,
-                             unsigned char* A) {
-  // zero the tile (padding rows and columns must not hold stale values)
-  for (int b = threadIdx.x * 16; b < 128 * KP * 2; b += kThreads * 16)
-    *reinterpret_cast<uint4*>(A + b) = make_uint4(0, 0, 0, 0);
-  __syncthreads();
-  const int Vh = G.g.Vh;
-  for (int j = threadIdx.x; j < kTileSites * 9; j += kThreads) {
-    const int sl = j / 9, d = j - sl * 9;
-    const int s = site0 + sl;
-    if (s >= G.V) continue;
-    const int p = s >= Vh ? 1 : 0;
-    const int hs = s - p * Vh;
-    int src = s;
-    Su3<float> U;
-    bool fwd = true;
-    if (d > 0) {
-      const Coord c = coord_of(G.g, hs, p);
-      int nb[8];
-      neighbours(G.g, c, hs, nb);
-      const int mu = (d - 1) >> 1;
-      fwd = ((d - 1) & 1) == 0;
-      const int n = nb[d - 1];
-      src = (1 - p) * Vh + n;
-      if (fwd)
-        GaugeIO<PREC_SINGLE, 12>::load(G.gauge, p, mu, hs, U);
-      else
-        GaugeIO<PREC_SINGLE, 12>::load(G.gauge, 1 - p, mu, n, U);
-    }
-#pragma unroll 4
-    for (int i = 0; i < CIN; ++i) {
-      Cx<float> v[3], w[3];
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const float2 t = feat_get(in, src, i, a, G.V);
-        v[a] = {t.x, t.y};
-      }
-      if (d == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) w[a] = v[a];
-      } else if (fwd) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) w[a] = U.e[a][0] * v[0] + U.e[a][1] * v[1] + U.e[a][2] * v[2];
-      } else {
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-          w[a] = cj_mul(U.e[0][a], v[0]) + cj_mul(U.e[1][a], v[1]) + cj_mul(U.e[2][a], v[2]);
-      }
-      const int kre = (2 * d) * CIN + i, kim = (2 * d + 1) * CIN + i;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const int r = sl * 3 + a;
-        *reinterpret_cast<__nv_bfloat16*>(A + canon(r, kre, KP)) = __float2bfloat16_rn(w[a].re);
-        *reinterpret_cast<__nv_bfloat16*>(A + canon(r, kim, KP)) = __float2bfloat16_rn(w[a].im);
-      }
-    }
-  }
-}
-
-// Loads an N x K row-major BF16 matrix into the canonical K-major layout.
-template <int N, int K>
-__device__ void load_b(const __nv_bfloat16* __restrict__ B, unsigned char* Bs) {
-  for (int idx = threadIdx.x; idx < N * K; idx += kThreads) {
-    const int n = idx / K, k = idx - n * K;
-    *reinterpret_cast<__nv_bfloat16*>(Bs + canon(n, k, K)) = B[idx];
-  }
-}
 
 // Issues the K/16 MMAs of D = A B^T into TMEM, commits to the mbarrier and
 // waits (bounded).  Only warp 0 polls the barrier (the other warps wait at
@@ -301,10 +229,72 @@ __device__ bool mma_and_wait(const unsigned char* A, const unsigned char* B, uin
 }
 
 // ---- forward ----------------------------------------------------------------------
+// The CIN channel vectors of site s transported along displacement d, as
+// BF16 words: wre/wim[colour][q] hold the real/imaginary parts of channels
+// 2q, 2q+1.  Channels are handled in pairs in the packed FP32x2 arithmetic
+// (su3_row).
+template <int CIN>
+__device__ __forceinline__ void transport_words(const PtcGeo& G, const float2* __restrict__ in, int s,
+                                                int d, uint32_t wre[3][CIN / 2],
+                                                uint32_t wim[3][CIN / 2]) {
+  constexpr int NW = CIN / 2;
+  const int Vh = G.g.Vh;
+  const int p = s >= Vh ? 1 : 0;
+  const int hs = s - p * Vh;
+  int src = s;
+  Su3<float> U;
+  bool fwd = true;
+  int mu = 0, n = hs;
+  if (d > 0) {
+    const Coord c = coord_of(G.g, hs, p);
+    int nb[8];
+    neighbours(G.g, c, hs, nb);
+    mu = (d - 1) >> 1;
+    fwd = ((d - 1) & 1) == 0;
+    n = nb[d - 1];
+    src = (1 - p) * Vh + n;
+  }
+  // channels 2q, 2q+1 of the source site, one float4 row per colour (see fidx)
+  const float4* f4 = reinterpret_cast<const float4*>(in) + src;
+  const size_t V = size_t(G.V);
+  // all of the job's feature rows requested at once (into L1), so that the
+  // loads below, which the register budget spreads over the channel
+  // pairs, find them there instead of each pair waiting on memory
+#pragma unroll
+  for (int q = 0; q < 3 * NW; ++q) asm volatile("prefetch.global.L1 [%0];" ::"l"(f4 + q * V));
+  if (d > 0) {
+    if (fwd)
+      GaugeIO<PREC_SINGLE, 12>::load(G.gauge, p, mu, hs, U);
+    else
+      GaugeIO<PREC_SINGLE, 12>::load(G.gauge, 1 - p, mu, n, U);
+  }
+#pragma unroll
+  for (int q = 0; q < NW; ++q) {
+    const float4 a = __ldg(f4 + (3 * q) * V), b = __ldg(f4 + (3 * q + 1) * V),
+                 e = __ldg(f4 + (3 * q + 2) * V);
+    const Cp h0 = {make_float2(a.x, a.y), make_float2(a.z, a.w)};
+    const Cp h1 = {make_float2(b.x, b.y), make_float2(b.z, b.w)};
+    const Cp h2 = {make_float2(e.x, e.y), make_float2(e.z, e.w)};
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      Cp w;
+      if (d == 0)
+        w = r == 0 ? h0 : (r == 1 ? h1 : h2);
+      else if (fwd)
+        w = su3_row<false>(U, r, h0, h1, h2);
+      else
+        w = su3_row<true>(U, r, h0, h1, h2);
+      const __nv_bfloat162 br = __floats2bfloat162_rn(w.re.x, w.re.y);
+      const __nv_bfloat162 bi = __floats2bfloat162_rn(w.im.x, w.im.y);
+      wre[r][q] = *reinterpret_cast<const uint32_t*>(&br);
+      wim[r][q] = *reinterpret_cast<const uint32_t*>(&bi);
+    }
+  }
+}
+
 // Writes the A-tile entries of one (site, displacement) job: the CIN
 // transported channel vectors of the tile's site sl, as BF16 in columns
-// (2d + re/im)*CIN + i of rows 3*sl + colour.  Channels are handled in pairs
-// in the packed FP32x2 arithmetic (su3_row); each colour row receives CIN/8
+// (2d + re/im)*CIN + i of rows 3*sl + colour; each colour row receives CIN/8
 // 16-byte stores (8-byte stores for CIN = 4).
 template <int CIN, int KP>
 __device__ __forceinline__ void a_tile_job(const PtcGeo& G, const float2* __restrict__ in, int s,
@@ -312,58 +302,7 @@ __device__ __forceinline__ void a_tile_job(const PtcGeo& G, const float2* __rest
   constexpr int NW = CIN / 2;  // BF16x2 words per colour and part
   uint32_t wre[3][NW], wim[3][NW];
   if (s < G.V) {
-    const int Vh = G.g.Vh;
-    const int p = s >= Vh ? 1 : 0;
-    const int hs = s - p * Vh;
-    int src = s;
-    Su3<float> U;
-    bool fwd = true;
-    int mu = 0, n = hs;
-    if (d > 0) {
-      const Coord c = coord_of(G.g, hs, p);
-      int nb[8];
-      neighbours(G.g, c, hs, nb);
-      mu = (d - 1) >> 1;
-      fwd = ((d - 1) & 1) == 0;
-      n = nb[d - 1];
-      src = (1 - p) * Vh + n;
-    }
-    // channels 2q, 2q+1 of the source site, one float4 row per colour (see fidx)
-    const float4* f4 = reinterpret_cast<const float4*>(in) + src;
-    const size_t V = size_t(G.V);
-    // all of the job's feature rows requested at once (into L1), so that the
-    // loads below, which the register budget spreads over the channel
-    // pairs, find them there instead of each pair waiting on memory
-#pragma unroll
-    for (int q = 0; q < 3 * NW; ++q) asm volatile("prefetch.global.L1 [%0];" ::"l"(f4 + q * V));
-    if (d > 0) {
-      if (fwd)
-        GaugeIO<PREC_SINGLE, 12>::load(G.gauge, p, mu, hs, U);
-      else
-        GaugeIO<PREC_SINGLE, 12>::load(G.gauge, 1 - p, mu, n, U);
-    }
-#pragma unroll
-    for (int q = 0; q < NW; ++q) {
-      const float4 a = __ldg(f4 + (3 * q) * V), b = __ldg(f4 + (3 * q + 1) * V),
-                   e = __ldg(f4 + (3 * q + 2) * V);
-      const Cp h0 = {make_float2(a.x, a.y), make_float2(a.z, a.w)};
-      const Cp h1 = {make_float2(b.x, b.y), make_float2(b.z, b.w)};
-      const Cp h2 = {make_float2(e.x, e.y), make_float2(e.z, e.w)};
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        Cp w;
-        if (d == 0)
-          w = r == 0 ? h0 : (r == 1 ? h1 : h2);
-        else if (fwd)
-          w = su3_row<false>(U, r, h0, h1, h2);
-        else
-          w = su3_row<true>(U, r, h0, h1, h2);
-        const __nv_bfloat162 br = __floats2bfloat162_rn(w.re.x, w.re.y);
-        const __nv_bfloat162 bi = __floats2bfloat162_rn(w.im.x, w.im.y);
-        wre[r][q] = *reinterpret_cast<const uint32_t*>(&br);
-        wim[r][q] = *reinterpret_cast<const uint32_t*>(&bi);
-      }
-    }
+    transport_words<CIN>(G, in, s, d, wre, wim);
   } else {
 #pragma unroll
     for (int r = 0; r < 3; ++r)
@@ -587,143 +526,190 @@ __global__ void __launch_bounds__(kFwdThreads, (CIN <= 4 ? 4 : (CIN <= 8 ? 3 : 1
   if (warp == 0) tmem_dealloc(tmem0, 2 * S::TCOLS);
 }
 
-// ---- backward: dA = dY B, stored as FP32 rows (site, colour) x KP ------------------
+// ---- backward: dB[n][k] = sum over rows (site, colour) of dY[row][n] A[row][k] ------
+// ldmatrix, four 8x8 BF16 matrices transposed: lane l gives the address of row
+// l % 8 of matrix l / 8
+__device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t r[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void ldsm2_t(uint32_t addr, uint32_t r[2]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1])
+               : "r"(addr)
+               : "memory");
+}
+// c (16x8, FP32) += a (16x16) b (16x8), BF16
+__device__ __forceinline__ void mma_16816(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Weight gradient of a layer.  Persistent CTAs of 9 warps loop over tiles of
+// 32 sites.  Warp d transports the tile's input channels along displacement d
+// (as the forward kernel) and multiplies its own 2*CIN columns of A with the
+// tile's dY: per colour, the 32 sites are the contraction index of two
+// m16n8k16 steps, M = the layer's real outputs, N = the warp's columns.  dY
+// stays FP32 in value: it is staged as three BF16 terms (hi + mid + lo, 24
+// bits), each multiplied with A and summed in FP32.  The accumulators live in
+// registers over all of a CTA's tiles, so a CTA writes one partial of dB; the
+// sum over CTAs is in block order.
+//
+// What bounds it is the transport (the gathers), as in the forward kernel;
+// the contraction takes 144 MMAs a warp and tile.  Before, each 42-site tile
+// was multiplied on the CUDA cores from shared memory and wrote its own
+// partial.  A 16->16 layer at 16^3x32: 2.33 ms before, 0.147 ms
+// now (and the input gradient, a product stored as FP32 rows and gathered back,
+// 2.30 ms, is a 0.109 ms forward layer).
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads) ptc_da_kernel(PtcGeo G, const float2* __restrict__ dy,
-                                                          float* __restrict__ da,
-                                                          const __nv_bfloat16* __restrict__ bopT) {
-  using S = Ptc<CIN, COUT>;
-  // operand A' = dY tile: 128 rows x NP (K' = NP); operand B' = B^T: KP rows x NP
-  constexpr int NCH = S::KP <= 256 ? S::KP : S::KP / 2;  // output columns per MMA pass
-  static_assert(NCH % 16 == 0 && NCH <= 256, "bad pass width");
-  constexpr int NPASS = S::KP / NCH;
-  constexpr int TC = NCH <= 32 ? 32 : (NCH <= 64 ? 64 : (NCH <= 128 ? 128 : 256));
+struct PtcDb {
+  static constexpr int NF = 2 * COUT;
+  static constexpr int MT = (NF + 15) / 16;      // 16-row output tiles
+  static constexpr int CH = CIN < 8 ? CIN : 8;    // channels transported at a time (registers)
+  static constexpr int NH = CIN / CH;
+  static constexpr int KC = 2 * CH;               // columns staged at a time: re, then im
+  static constexpr int NT = KC / 8;               // their 8-column tiles
+  static constexpr int YS = MT * 32 + 16;         // bytes of a dY row (padded: conflict-free ldmatrix)
+  static constexpr int AS = NT == 1 ? 16 : 48;    // bytes of an A row (as above)
+  static constexpr int Y_BYTES = 96 * YS;         // one split of one tile
+  static constexpr int A_BYTES = 32 * AS;         // one colour of one warp
+  static constexpr int SMEM = 2 * 3 * Y_BYTES + 9 * A_BYTES;
+};
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kFwdThreads, 2) ptc_db_kernel(PtcGeo G, const float2* __restrict__ in,
+                                                             const float2* __restrict__ dy,
+                                                             float* __restrict__ partial, int ntiles) {
+  using S = PtcDb<CIN, COUT>;
+  constexpr int NW = S::CH / 2;
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char* A = smem;                 // 128 x NP
-  unsigned char* B = smem + 128 * S::NP * 2;  // KP x NP
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ uint32_t tslot;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) tmem_alloc(&tslot, TC);
-  if (threadIdx.x == 0) mbar_init(&bar, 1);
-  load_b<S::KP, S::NP>(bopT, B);
-  const int site0 = blockIdx.x * kTileSites;
-  for (int idx = threadIdx.x; idx < 128 * S::NP; idx += kThreads) {
-    const int r = idx / S::NP, n = idx - r * S::NP;
-    const int sl = r / 3, a = r - sl * 3, s = site0 + sl;
-    float val = 0.f;
-    if (sl < kTileSites && s < G.V && n < S::NF) {
-      const float2 t = feat_get(dy, s, n >> 1, a, G.V);
-      val = (n & 1) ? t.y : t.x;
-    }
-    *reinterpret_cast<__nv_bfloat16*>(A + canon(r, n, S::NP)) = __float2bfloat16_rn(val);
-  }
-  tc_fence_before();
+  unsigned char* As = smem + 6 * S::Y_BYTES + warp * S::A_BYTES;
+  // the padding columns of dY (COUT = 4: 8 of 16) stay zero
+  for (int b = threadIdx.x * 16; b < 6 * S::Y_BYTES; b += kFwdThreads * 16)
+    *reinterpret_cast<uint4*>(smem + b) = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tslot;
-  const int r = warp * 32 + lane;
-  const int sl = r / 3, a = r - sl * 3, s = site0 + sl;
-  for (int pass = 0; pass < NPASS; ++pass) {
-    const bool ok = mma_and_wait<S::NP>(A, B + pass * NCH * S::NP * 2 / 1, tmem, idesc_bf16(NCH), &bar,
-                                        uint32_t(pass & 1), G.err);
-    if (!ok) break;
-    float v[16];
-    for (int c = 0; c < NCH; c += 16) {
-      tmem_ld16(tmem + (uint32_t(warp * 32) << 16) + c, v);
-      if (sl < kTileSites && s < G.V) {
+  float acc[S::MT][S::NH * S::NT][4];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) da[(size_t(s) * 3 + a) * S::KP + pass * NCH + c + k] = v[k];
+  for (int m = 0; m < S::MT; ++m)
+#pragma unroll
+    for (int n = 0; n < S::NH * S::NT; ++n)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[m][n][k] = 0.f;
+  // ldmatrix addresses of this lane: matrix j = lane / 8 of dY covers rows
+  // 8 (j / 2) and columns 8 (j % 2), of A rows 8 (j % 2) and columns 8 (j / 2)
+  const int lj = lane >> 3, lr = lane & 7;
+  const uint32_t y_off = uint32_t((8 * (lj >> 1) + lr) * S::YS + 16 * (lj & 1));
+  const uint32_t a_off = smem_u32(As) + uint32_t((8 * (lj & 1) + lr) * S::AS + 16 * (lj >> 1));
+  for (int tile = blockIdx.x, it = 0; tile < ntiles; tile += gridDim.x, ++it) {
+    const int site0 = fwd_tile_site0(G, tile);
+    unsigned char* Y = smem + (it & 1) * 3 * S::Y_BYTES;
+    // dY of the tile: float4 row (3q + colour) of 32 sites -> columns 4q .. 4q+3
+    // (re 2q, re 2q+1, im 2q, im 2q+1) of rows 32 colour + site
+    for (int j = threadIdx.x; j < 32 * 3 * (COUT / 2); j += kFwdThreads) {
+      const int sl = j & 31, qa = j >> 5;
+      const int q = qa / 3, a = qa - 3 * q;
+      const float4 v = __ldg(reinterpret_cast<const float4*>(dy) + size_t(qa) * G.V + site0 + sl);
+      float x[4] = {v.x, v.y, v.z, v.w};
+      unsigned char* row = Y + (32 * a + sl) * S::YS + 8 * q;
+#pragma unroll
+      for (int sp = 0; sp < 3; ++sp) {
+        const __nv_bfloat162 b01 = __floats2bfloat162_rn(x[0], x[1]);
+        const __nv_bfloat162 b23 = __floats2bfloat162_rn(x[2], x[3]);
+        *reinterpret_cast<uint2*>(row + sp * S::Y_BYTES) = make_uint2(
+            *reinterpret_cast<const uint32_t*>(&b01), *reinterpret_cast<const uint32_t*>(&b23));
+        const float2 f01 = __bfloat1622float2(b01), f23 = __bfloat1622float2(b23);
+        x[0] -= f01.x;
+        x[1] -= f01.y;
+        x[2] -= f23.x;
+        x[3] -= f23.y;
       }
     }
-    tc_fence_before();
-    __syncthreads();
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, TC);
-}
-
-// d in(y)_i = dA_0(y) + sum_mu U_mu(y-mu)^dag dA_{+mu}(y-mu) + U_mu(y) dA_{-mu}(y+mu)
-template <int CIN, int KP>
-__global__ void ptc_gather_kernel(PtcGeo G, const float* __restrict__ da, float2* __restrict__ din) {
-  const int Vh = G.g.Vh;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < G.V; s += gridDim.x * blockDim.x) {
-    const int p = s >= Vh ? 1 : 0;
-    const int hs = s - p * Vh;
-    const Coord c = coord_of(G.g, hs, p);
-    int nb[8];
-    neighbours(G.g, c, hs, nb);
-    for (int i = 0; i < CIN; ++i) {
-      Cx<float> acc[3];
-      auto grad = [&](int site, int d, Cx<float> g[3]) {
+    const uint32_t y0 = smem_u32(Y) + y_off;
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-          g[a] = {da[(size_t(site) * 3 + a) * KP + (2 * d) * CIN + i],
-                  da[(size_t(site) * 3 + a) * KP + (2 * d + 1) * CIN + i]};
-      };
-      grad(s, 0, acc);
-#pragma unroll 1
-      for (int mu = 0; mu < 4; ++mu) {
-        Cx<float> g[3];
-        Su3<float> U;
-        // from x = y - mu (d = +mu): U_mu(x)^dag g
-        const int xm = nb[2 * mu + 1];
-        grad((1 - p) * Vh + xm, 1 + 2 * mu, g);
-        GaugeIO<PREC_SINGLE, 12>::load(G.gauge, 1 - p, mu, xm, U);
+    for (int h = 0; h < S::NH; ++h) {
+      uint32_t wre[3][NW], wim[3][NW];
+      transport_words<S::CH>(G, in + size_t(24 * h) * G.V, site0 + lane, warp, wre, wim);
+      // one barrier a tile: the other dY buffer is written next, and this one
+      // again only after every warp has passed the next tile's barrier
+      if (h == 0) __syncthreads();
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-          acc[a] = acc[a] + cj_mul(U.e[0][a], g[0]) + cj_mul(U.e[1][a], g[1]) + cj_mul(U.e[2][a], g[2]);
-        // from x = y + mu (d = -mu): U_mu(y) g
-        const int xp = nb[2 * mu];
-        grad((1 - p) * Vh + xp, 2 + 2 * mu, g);
-        GaugeIO<PREC_SINGLE, 12>::load(G.gauge, p, mu, hs, U);
+      for (int a = 0; a < 3; ++a) {
+        __syncwarp();
+        unsigned char* row = As + lane * S::AS;
+        if constexpr (CIN == 4) {
+          *reinterpret_cast<uint4*>(row) = make_uint4(wre[a][0], wre[a][1], wim[a][0], wim[a][1]);
+        } else {
+          *reinterpret_cast<uint4*>(row) = make_uint4(wre[a][0], wre[a][1], wre[a][2], wre[a][3]);
+          *reinterpret_cast<uint4*>(row + 16) = make_uint4(wim[a][0], wim[a][1], wim[a][2], wim[a][3]);
+        }
+        __syncwarp();
 #pragma unroll
-        for (int a = 0; a < 3; ++a) acc[a] = acc[a] + U.e[a][0] * g[0] + U.e[a][1] * g[1] + U.e[a][2] * g[2];
+        for (int ks = 0; ks < 2; ++ks) {
+          uint32_t b[4];
+          if constexpr (S::NT == 1)
+            ldsm2_t(a_off + uint32_t(16 * ks * S::AS), b);
+          else
+            ldsm4_t(a_off + uint32_t(16 * ks * S::AS), b);
+#pragma unroll
+          for (int m = 0; m < S::MT; ++m)
+#pragma unroll
+            for (int sp = 2; sp >= 0; --sp) {
+              uint32_t ya[4];
+              ldsm4_t(y0 + uint32_t(sp * S::Y_BYTES + (32 * a + 16 * ks) * S::YS + 32 * m), ya);
+#pragma unroll
+              for (int n = 0; n < S::NT; ++n)
+                mma_16816(acc[m][h * S::NT + n], ya, b[2 * n], b[2 * n + 1]);
+            }
+        }
       }
+    }
+  }
+  // row n' = 4q + j of the accumulators is output n = 2o + re/im with
+  // o = 2q + (j & 1), re/im = j >> 1; the columns of tile (h, t) are the real
+  // (t = 0) or imaginary (t = 1) parts of channels 8h .. 8h + 7 (4 input
+  // channels: one tile, re then im), k = (2d + re/im) CIN + channel
+  constexpr int KF = 18 * CIN;
+  float* out = partial + size_t(blockIdx.x) * S::NF * KF + warp * 2 * CIN + 2 * (lane & 3);
 #pragma unroll
-      for (int a = 0; a < 3; ++a) feat_set(din, s, i, a, G.V, make_float2(acc[a].re, acc[a].im));
+  for (int m = 0; m < S::MT; ++m)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int np = 16 * m + 8 * h + (lane >> 2);
+      if (np < S::NF) {
+        const int n = 2 * (2 * (np >> 2) + (np & 1)) + ((np >> 1) & 1);
+#pragma unroll
+        for (int t = 0; t < S::NH * S::NT; ++t)
+          *reinterpret_cast<float2*>(out + size_t(n) * KF + (t % S::NT) * CIN + 8 * (t / S::NT)) =
+              make_float2(acc[m][t][2 * h], acc[m][t][2 * h + 1]);
+      }
     }
-  }
 }
 
-// dB[n][k] = sum_rows dY[row][n] A[row][k], one partial per tile (CUDA cores)
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads) ptc_db_kernel(PtcGeo G, const float2* __restrict__ in,
-                                                          const float2* __restrict__ dy,
-                                                          float* __restrict__ partial) {
-  using S = Ptc<CIN, COUT>;
-  extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char* A = smem;
-  float* Y = reinterpret_cast<float*>(smem + S::A_BYTES);  // 128 x NF
-  const int site0 = blockIdx.x * kTileSites;
-  build_a_tile<CIN, S::KP>(G, in, site0, A);
-  for (int idx = threadIdx.x; idx < 128 * S::NF; idx += kThreads) {
-    const int r = idx / S::NF, n = idx - r * S::NF;
-    const int sl = r / 3, a = r - sl * 3, s = site0 + sl;
-    float val = 0.f;
-    if (sl < kTileSites && s < G.V) {
-      const float2 t = feat_get(dy, s, n >> 1, a, G.V);
-      val = (n & 1) ? t.y : t.x;
-    }
-    Y[idx] = val;
+// Deterministic sum over the CTAs' partials: 8 threads take every 8th partial
+// of one entry, and their sums are added in order (one thread per entry kept
+// 36 blocks busy with a serial chain of loads over one partial per tile: 374 us
+// a call, 6 us now).
+constexpr int kSumSlices = 8;
+__global__ void __launch_bounds__(32 * kSumSlices) sum_partials_kernel(const float* __restrict__ partial,
+                                                                       int nparts, int n, float* out) {
+  __shared__ double sm[kSumSlices][32];
+  const int q = blockIdx.x * 32 + threadIdx.x, sl = threadIdx.y;
+  double acc = 0.0;
+  if (q < n) {
+#pragma unroll 8
+    for (int t = sl; t < nparts; t += kSumSlices) acc += double(__ldg(partial + size_t(t) * n + q));
   }
+  sm[sl][threadIdx.x] = acc;
   __syncthreads();
-  float* out = partial + size_t(blockIdx.x) * S::NF * S::KF;
-  for (int q = threadIdx.x; q < S::NF * S::KF; q += kThreads) {
-    const int n = q / S::KF, k = q - n * S::KF;
-    float acc = 0.f;
-    for (int r = 0; r < 126; ++r)
-      acc += Y[r * S::NF + n] * __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(A + canon(r, k, S::KP)));
-    out[q] = acc;
-  }
-}
-
-// deterministic sum over tiles
-__global__ void sum_partials_kernel(const float* __restrict__ partial, int ntiles, int n, float* out) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-    double acc = 0.0;
-    for (int t = 0; t < ntiles; ++t) acc += partial[size_t(t) * n + q];
+  if (sl == 0 && q < n) {
+#pragma unroll
+    for (int k = 1; k < kSumSlices; ++k) acc += sm[k][threadIdx.x];
     out[q] = float(acc);
   }
 }
@@ -826,51 +812,31 @@ static cudaError_t fwd_t(const PtcGeo& G, const float2* in, float2* out, const _
   return cudaGetLastError();
 }
 
+// CTAs of the weight-gradient kernel (its partial buffer holds as many)
+static int db_grid(int V) {
+  const int ntiles = (V + kFwdSites - 1) / kFwdSites;
+  return std::min(ntiles, 2 * sm_count());
+}
+
 template <int CIN, int COUT>
-static cudaError_t bwd_t(const PtcGeo& G, const float2* in, const float2* dy, float* da, float2* din,
-                         const __nv_bfloat16* bopT, float* partial, float* db, cudaStream_t st) {
-  using S = Ptc<CIN, COUT>;
-  const int grid = (G.V + kTileSites - 1) / kTileSites;
-  if (din) {
-    // the pass accumulator takes up to 256 TMEM columns: ask for enough shared
-    // memory that at most two CTAs share an SM (2 x 256 = its 512 columns),
-    // so tensor-memory allocation never has to wait
-    constexpr int NCH = S::KP <= 256 ? S::KP : S::KP / 2;
-    constexpr int TC = NCH <= 32 ? 32 : (NCH <= 64 ? 64 : (NCH <= 128 ? 128 : 256));
-    const int need = 128 * S::NP * 2 + S::KP * S::NP * 2;
-    const int cap = TC >= 256 ? 100 * 1024 : (TC >= 128 ? 52 * 1024 : 0);
-    const int smem = need > cap ? need : cap;
-    static bool attr = false;
-    if (!attr) {
-      cudaError_t e = cudaFuncSetAttribute(ptc_da_kernel<CIN, COUT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return e;
-      attr = true;
-    }
-    ptc_da_kernel<CIN, COUT><<<grid, kThreads, smem, st>>>(G, dy, da, bopT);
-    cudaError_t e = cudaGetLastError();
+static cudaError_t db_t(const PtcGeo& G, const float2* in, const float2* dy, float* partial, float* db,
+                        cudaStream_t st) {
+  using S = PtcDb<CIN, COUT>;
+  static bool attr = false;
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(ptc_db_kernel<CIN, COUT>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
     if (e != cudaSuccess) return e;
-    ptc_gather_kernel<CIN, S::KP><<<(G.V + 255) / 256, 256, 0, st>>>(G, da, din);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    attr = true;
   }
-  if (db) {
-    const int smem = S::A_BYTES + 128 * S::NF * 4;
-    static bool attr = false;
-    if (!attr) {
-      cudaError_t e = cudaFuncSetAttribute(ptc_db_kernel<CIN, COUT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return e;
-      attr = true;
-    }
-    ptc_db_kernel<CIN, COUT><<<grid, kThreads, smem, st>>>(G, in, dy, partial);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    sum_partials_kernel<<<(S::NF * S::KF + 255) / 256, 256, 0, st>>>(partial, grid, S::NF * S::KF, db);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  const int grid = db_grid(G.V);
+  ptc_db_kernel<CIN, COUT><<<grid, kFwdThreads, S::SMEM, st>>>(G, in, dy, partial,
+                                                               (G.V + kFwdSites - 1) / kFwdSites);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const int n = S::NF * 18 * CIN;
+  sum_partials_kernel<<<(n + 31) / 32, dim3(32, kSumSlices), 0, st>>>(partial, grid, n, db);
+  return cudaGetLastError();
 }
 
 int ptc_shape_ok(int cin, int cout) {
@@ -898,10 +864,9 @@ cudaError_t launch_ptc_fwd(int cin, int cout, const PtcGeo& G, const float2* in,
 #undef IRO_F
 }
 
-cudaError_t launch_ptc_bwd(int cin, int cout, const PtcGeo& G, const float2* in, const float2* dy,
-                           float* da, float2* din, const void* bopT, float* partial, float* db,
-                           cudaStream_t st) {
-#define IRO_B(A, B) bwd_t<A, B>(G, in, dy, da, din, static_cast<const __nv_bfloat16*>(bopT), partial, db, st)
+cudaError_t launch_ptc_db(int cin, int cout, const PtcGeo& G, const float2* in, const float2* dy,
+                          float* partial, float* db, cudaStream_t st) {
+#define IRO_B(A, B) db_t<A, B>(G, in, dy, partial, db, st)
   IRO_PTC_DISPATCH(IRO_B)
 #undef IRO_B
 }
@@ -1361,13 +1326,12 @@ struct iro_ptc {
   int nl = 0;
   std::vector<int> w;                 // widths, nl+1 entries
   std::vector<std::vector<float>> W;  // host weights, complex [9][cout][cin] (re,im)
-  std::vector<void*> bop, bopT;       // device BF16 packed weights per layer
+  std::vector<void*> bop, badj;       // device BF16 packed weights per layer, and its adjoint's
   std::vector<float2*> act;           // act[l]: input of layer l (act[nl]: output)
   float2* g0 = nullptr;               // gradient ping-pong buffers
   float2* g1 = nullptr;
-  float* da = nullptr;
-  float* partial = nullptr;
-  std::vector<float*> db;
+  float* partial = nullptr;           // weight-gradient partials, one per CTA
+  float* db = nullptr;                // every layer's dL/dB, consecutive
   int* err = nullptr;
   double* lpart = nullptr;
   size_t maxc = 0;
@@ -1375,8 +1339,7 @@ struct iro_ptc {
 
 namespace {
 
-void pack_bop(int cin, int cout, const std::vector<float>& W, std::vector<__nv_bfloat16>& bop,
-              std::vector<__nv_bfloat16>& bopT) {
+void pack_bop(int cin, int cout, const std::vector<float>& W, std::vector<__nv_bfloat16>& bop) {
   int kf, kp, nf, np;
   ptc_dims(cin, cout, &kf, &kp, &nf, &np);
   std::vector<float> B(size_t(np) * kp, 0.f);
@@ -1392,16 +1355,29 @@ void pack_bop(int cin, int cout, const std::vector<float>& W, std::vector<__nv_b
         B[size_t(2 * o + 1) * kp + kim] = wr;
       }
   bop.resize(B.size());
-  bopT.resize(B.size());
-  for (int n = 0; n < np; ++n)
-    for (int k = 0; k < kp; ++k) {
-      bop[size_t(n) * kp + k] = __float2bfloat16_rn(B[size_t(n) * kp + k]);
-      bopT[size_t(k) * np + n] = __float2bfloat16_rn(B[size_t(n) * kp + k]);
-    }
+  for (size_t k = 0; k < B.size(); ++k) bop[k] = __float2bfloat16_rn(B[k]);
+}
+
+// The adjoint layer's weights [9][cin][cout]: with y = sum_d W_d T_d x the
+// gradient of x is sum_d W_d^dag T_d^dag dy, and T_{+mu}^dag = T_{-mu}, so it is
+// a layer on dy whose displacement d has the weights of the opposite one,
+// conjugate transposed.
+std::vector<float> adjoint_weights(int cin, int cout, const std::vector<float>& W) {
+  std::vector<float> A(W.size());
+  for (int d = 0; d < 9; ++d) {
+    const int e = d == 0 ? 0 : ((d - 1) ^ 1) + 1;
+    for (int o = 0; o < cout; ++o)
+      for (int i = 0; i < cin; ++i) {
+        const size_t w = ((size_t(e) * cout + o) * cin + i) * 2, a = ((size_t(d) * cin + i) * cout + o) * 2;
+        A[a] = W[w];
+        A[a + 1] = -W[w + 1];
+      }
+  }
+  return A;
 }
 
 // dL/dB (NF x KF, real) -> dL/dW (complex [9][cout][cin])
-void unpack_grad(int cin, int cout, const std::vector<float>& dB, float* g) {
+void unpack_grad(int cin, int cout, const float* dB, float* g) {
   int kf, kp, nf, np;
   ptc_dims(cin, cout, &kf, &kp, &nf, &np);
   for (int d = 0; d < 9; ++d)
@@ -1496,27 +1472,28 @@ int iro_ptc_create(iro_ctx* c, int nlayers, const int* widths, iro_ptc** out) {
   n->maxc = maxc;
   n->W.resize(nlayers);
   n->bop.resize(nlayers);
-  n->bopT.resize(nlayers);
-  n->db.resize(nlayers);
+  n->badj.resize(nlayers);
   n->act.resize(nlayers + 1);
-  int maxkp = 0, maxtiles = int((V + kTileSites - 1) / kTileSites), maxnk = 0;
+  int maxnk = 0;
+  size_t gradn = 0;
   for (int l = 0; l < nlayers; ++l) {
     int kf, kp, nf, np;
     ptc_dims(n->w[l], n->w[l + 1], &kf, &kp, &nf, &np);
-    maxkp = std::max(maxkp, kp);
+    gradn += size_t(nf) * kf;
     maxnk = std::max(maxnk, nf * kf);
     n->W[l].assign(size_t(9) * n->w[l + 1] * n->w[l] * 2, 0.f);
     LCK(cudaMalloc(&n->bop[l], size_t(np) * kp * 2));
-    LCK(cudaMalloc(&n->bopT[l], size_t(np) * kp * 2));
+    int akf, akp, anf, anp;
+    ptc_dims(n->w[l + 1], n->w[l], &akf, &akp, &anf, &anp);
+    LCK(cudaMalloc(&n->badj[l], size_t(anp) * akp * 2));
     LCK(cudaMemset(n->bop[l], 0, size_t(np) * kp * 2));
-    LCK(cudaMemset(n->bopT[l], 0, size_t(np) * kp * 2));
-    LCK(cudaMalloc(&n->db[l], size_t(nf) * kf * sizeof(float)));
+    LCK(cudaMemset(n->badj[l], 0, size_t(anp) * akp * 2));
   }
   for (int l = 0; l <= nlayers; ++l) LCK(cudaMalloc(&n->act[l], V * n->w[l] * 3 * sizeof(float2)));
   LCK(cudaMalloc(&n->g0, V * maxc * 3 * sizeof(float2)));
   LCK(cudaMalloc(&n->g1, V * maxc * 3 * sizeof(float2)));
-  LCK(cudaMalloc(&n->da, V * 3 * maxkp * sizeof(float)));
-  LCK(cudaMalloc(&n->partial, size_t(maxtiles) * maxnk * sizeof(float)));
+  LCK(cudaMalloc(&n->db, gradn * sizeof(float)));
+  LCK(cudaMalloc(&n->partial, size_t(db_grid(int(V))) * maxnk * sizeof(float)));
   LCK(cudaMalloc(&n->err, sizeof(int)));
   LCK(cudaMemset(n->err, 0, sizeof(int)));
   LCK(cudaMalloc(&n->lpart, sizeof(double) * 2 * loss_blocks()));
@@ -1529,10 +1506,9 @@ int iro_ptc_destroy(iro_ptc* n) {
   // cudaFree waits for the device's work on these buffers; the context may be gone
   cudaSetDevice(n->dev);
   for (void* p : n->bop) cudaFree(p);
-  for (void* p : n->bopT) cudaFree(p);
-  for (float* p : n->db) cudaFree(p);
+  for (void* p : n->badj) cudaFree(p);
   for (float2* p : n->act) cudaFree(p);
-  void* ps[] = {n->g0, n->g1, n->da, n->partial, n->err, n->lpart};
+  void* ps[] = {n->g0, n->g1, n->db, n->partial, n->err, n->lpart};
   for (void* p : ps)
     if (p) cudaFree(p);
   delete n;
@@ -1546,9 +1522,10 @@ int iro_ptc_set_weights(iro_ptc* n, int layer, const float* w) {
   const int cin = n->w[layer], cout = n->w[layer + 1];
   n->W[layer].assign(w, w + size_t(9) * cout * cin * 2);
   std::vector<__nv_bfloat16> b, bt;
-  pack_bop(cin, cout, n->W[layer], b, bt);
+  pack_bop(cin, cout, n->W[layer], b);
+  pack_bop(cout, cin, adjoint_weights(cin, cout, n->W[layer]), bt);
   LCK(cudaMemcpyAsync(n->bop[layer], b.data(), b.size() * 2, cudaMemcpyHostToDevice, stream(c)));
-  LCK(cudaMemcpyAsync(n->bopT[layer], bt.data(), bt.size() * 2, cudaMemcpyHostToDevice, stream(c)));
+  LCK(cudaMemcpyAsync(n->badj[layer], bt.data(), bt.size() * 2, cudaMemcpyHostToDevice, stream(c)));
   LCK(cudaStreamSynchronize(stream(c)));
   return IRO_OK;
 }
@@ -1624,20 +1601,21 @@ int iro_ptc_loss_grad(iro_ctx* c, iro_ptc* n, const iro_field* in, const iro_fie
   PtcGeo G = make_geo(c, n->err);
   float2* dy = n->g0;
   float2* dx = n->g1;
-  std::vector<size_t> goff(n->nl + 1, 0);
-  for (int l = 0; l < n->nl; ++l) goff[l + 1] = goff[l] + size_t(9) * n->w[l + 1] * n->w[l] * 2;
+  std::vector<size_t> goff(n->nl + 1, 0), boff(n->nl + 1, 0);
+  for (int l = 0; l < n->nl; ++l) {
+    goff[l + 1] = goff[l] + size_t(9) * n->w[l + 1] * n->w[l] * 2;
+    boff[l + 1] = boff[l] + size_t(18) * n->w[l] * 2 * n->w[l + 1];
+  }
   for (int l = n->nl - 1; l >= 0; --l) {
     const int cin = n->w[l], cout = n->w[l + 1];
-    LCK(launch_ptc_bwd(cin, cout, G, n->act[l], dy, n->da, l > 0 ? dx : nullptr, n->bopT[l],
-                       n->partial, n->db[l], st));
-    int kf, kp, nf, np;
-    ptc_dims(cin, cout, &kf, &kp, &nf, &np);
-    std::vector<float> dB(size_t(nf) * kf);
-    LCK(cudaMemcpyAsync(dB.data(), n->db[l], dB.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
-    LCK(cudaStreamSynchronize(st));
-    unpack_grad(cin, cout, dB, grad + goff[l]);
+    LCK(launch_ptc_db(cin, cout, G, n->act[l], dy, n->partial, n->db + boff[l], st));
+    if (l > 0) LCK(launch_ptc_fwd(cout, cin, G, dy, dx, n->badj[l], st));
     std::swap(dy, dx);
   }
+  std::vector<float> dB(boff[n->nl]);
+  LCK(cudaMemcpyAsync(dB.data(), n->db, dB.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
+  LCK(cudaStreamSynchronize(st));
+  for (int l = 0; l < n->nl; ++l) unpack_grad(n->w[l], n->w[l + 1], dB.data() + boff[l], grad + goff[l]);
   return check_err(c, n);
 }
 

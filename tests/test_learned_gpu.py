@@ -57,6 +57,29 @@ def test_loss_and_gradients_vs_oracle(small):
         assert rel(g, go) < 5e-2
 
 
+@pytest.mark.parametrize("widths", [(4, 4), (4, 8, 4), (4, 4, 16, 4), (4, 8, 8, 16, 8, 4)])
+def test_gradients_of_every_layer_shape(widths):
+    """Each weight-gradient kernel (4, 8 and 16 channels in and out) and each
+    adjoint layer, on a lattice of a few tiles (fewer than the CTAs of a
+    launch) and of an odd number of tiles per CTA."""
+    L = [4, 6, 4, 14]
+    V = int(np.prod(L))
+    u = ib.synth_gauge(L, 0.25, 23, gauge_transform=True)
+    ctx = ib.Context(L, 0)
+    ctx.upload_gauge(u, force=True)
+    Ws = learned.init_weights(widths, seed=6, scale=0.5)
+    net = learned.PTCNet(ctx, widths, Ws)
+    b, t = ib.synth_gaussian(V, 43), ib.synth_gaussian(V, 44)
+    db = ib.DeviceField(ctx, 2, "double").upload(b)
+    dt = ib.DeviceField(ctx, 2, "double").upload(t)
+    loss, grads = net.loss_grad(ctx, db, dt)
+    lat = ptc.Lattice(L, u)
+    loss_o, grads_o, _ = ptc.loss_grad(lat, Ws, ptc.spinor_to_feat(lat, b), ptc.spinor_to_feat(lat, t))
+    assert abs(loss - loss_o) < TOL_NET * loss_o
+    for g, go in zip(grads, grads_o):
+        assert rel(g, go) < 5e-2  # BF16 operands through every layer and back
+
+
 def _pair(L, seed):
     u = ib.synth_gauge(L, 0.2, seed)
     ctx = ib.Context(L, 0)
