@@ -597,7 +597,7 @@ int clover_build(iro_ctx* c, double kc) {
       ca.Ainv[pr][p] = c->clAinv[pr][p];
     }
   CK(cudaMemsetAsync(c->d_singular, 0, sizeof(int), c->stream));
-  CK(launch_clover_build(c->g, c->raw, kc, ca, c->d_singular, c->stream));
+  CK(launch_clover_build(c->g, c->ga.d18, kc, ca, c->d_singular, c->stream));
   int singular = 0;
   CK(cudaMemcpyAsync(&singular, c->d_singular, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -720,7 +720,6 @@ int iro_ctx_create(const int L[4], int device, iro_ctx** out) {
     CK(cudaMallocHost(&c->h_pinned, 4096 + sizeof(MSState)));
     CK(cudaMalloc(&c->d_maxdev, sizeof(unsigned long long)));
     CK(cudaMalloc(&c->d_singular, sizeof(int)));
-    clover_init_tables();
     CK(cudaGetLastError());
   }
   *out = c.release();
@@ -832,7 +831,7 @@ int iro_field_strength(iro_ctx* c, int mu, int nu, double* out) {
   const size_t bytes = size_t(18) * c->V * sizeof(double);
   int rc = ensure_stage(c, bytes);
   if (rc) return rc;
-  CK(launch_field_strength(c->g, c->raw, mu, nu, c->stage, c->stream));
+  CK(launch_field_strength(c->g, c->ga.d18, mu, nu, c->stage, c->stream));
   return copy_d2h(c, out, c->stage, bytes);
 }
 
@@ -1256,7 +1255,7 @@ bool op_ok(int op) { return op_valid(op); }
 int clover_ready(iro_ctx* c, double mass, double csw) { return ensure_clover(c, mass, csw); }
 GaugePtr gauge_double(iro_ctx* c) { return gauge_ptr(c, PREC_DOUBLE); }
 int gauge_recon(iro_ctx* c) { return c->recon; }
-const double* gauge_format_g(iro_ctx* c) { return c->raw; }
+const double2* gauge_d18(iro_ctx* c) { return c->ga.d18; }
 bool gauge_loaded(iro_ctx* c) { return c->has_gauge; }
 CloverPtr clover(iro_ctx* c, int prec, int p, bool inverse) { return clover_ptr(c, prec, p, inverse); }
 }  // namespace host

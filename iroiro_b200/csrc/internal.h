@@ -189,16 +189,20 @@ struct GaugeArrays {
 cudaError_t launch_import_gauge(const Geom& g, const double* raw, GaugeArrays ga,
                                 unsigned long long* maxdev_bits, cudaStream_t st);
 
-// ---- clover ------------------------------------------------------------------------
+// ---- clover (clover.cu) ------------------------------------------------------------
 struct CloverArrays {
   void* A[3][2];     // [prec][parity]
   void* Ainv[3][2];
 };
-cudaError_t launch_clover_build(const Geom& g, const double* raw, double kappa_csw,
+// from the FP64 links with three stored rows (GaugeArrays::d18)
+cudaError_t launch_clover_build(const Geom& g, const double2* d18, double kappa_csw,
                                 CloverArrays ca, int* singular, cudaStream_t st);
-cudaError_t launch_field_strength(const Geom& g, const double* raw, int mu, int nu, double* out,
+// the clover block of Dirac_Clover::md_force, added to F (Format_G) with weight
+// w = -kappa csw / 4; lam: scratch of 6 * 9 * V doubles
+cudaError_t launch_clover_force(const Geom& g, const double2* d18, SpinorPtr e0, SpinorPtr e1, SpinorPtr z0,
+                                SpinorPtr z1, double w, double* lam, double* F, cudaStream_t st);
+cudaError_t launch_field_strength(const Geom& g, const double2* d18, int mu, int nu, double* out,
                                   cudaStream_t st);
-void clover_init_tables();
 
 // ---- rational-function reconstruction and clover fields (kernels.cu) --------------
 constexpr int kMaxCombine = 16;
@@ -216,11 +220,6 @@ cudaError_t launch_clover_mult(int64_t Vh, int nrhs, CloverPtr cl, SpinorPtr in,
 // ---- molecular-dynamics force (forces.cu) ------------------------------------------
 // F[mu][lex site][18] += w (1 - g_mu) U_mu(x) psi(x+mu) (x) chi(x)^dag over the
 // sites x of parity p (gamma5 on both fields when g5)
-// the clover block of Dirac_Clover::md_force, added to F (Format_G) with weight
-// w = -kappa csw / 4; lam: scratch of 6 * 9 * V double2
-cudaError_t launch_clover_force(const Geom& g, const double* u_format_g, SpinorPtr e0, SpinorPtr e1,
-                                SpinorPtr z0, SpinorPtr z1, double w, double2* lam, double* F,
-                                cudaStream_t st);
 cudaError_t launch_force(const Geom& g, const GaugePtr& gauge, int recon, int p, SpinorPtr psi,
                          SpinorPtr chi, int g5, double w, double* F, cudaStream_t st);
 

@@ -907,272 +907,6 @@ cudaError_t launch_import_gauge(const Geom& g, const double* raw, GaugeArrays ga
   return cudaGetLastError();
 }
 
-// ---- clover set-up (FP64) -------------------------------------------------------------
-// Spin matrices i*sigma_{mu nu} of Dirac_Clover::isigma_{23,31,12,41,42,43}
-// (lib/Dirac_ops/dirac_clover.cpp:221-329) reduced to the two chirality
-// blocks: s_pm[k][a][b] = S_k[a][b] +- S_k[a][b+2] for a,b in {0,1}.
-__constant__ double2 c_spm[2][6][2][2];
-
-struct M3d {
-  Cx<double> e[3][3];
-};
-
-__device__ __forceinline__ M3d m3_load(const double* raw, int64_t V, int64_t site, int mu) {
-  M3d m;
-  const double* u = raw + 18 * (site + V * mu);
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) m.e[a][b] = {u[2 * (3 * a + b)], u[2 * (3 * a + b) + 1]};
-  return m;
-}
-__device__ __forceinline__ M3d m3_mul(const M3d& x, const M3d& y) {
-  M3d r;
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) r.e[a][b] = x.e[a][0] * y.e[0][b] + x.e[a][1] * y.e[1][b] + x.e[a][2] * y.e[2][b];
-  return r;
-}
-__device__ __forceinline__ M3d m3_dag(const M3d& x) {
-  M3d r;
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) r.e[a][b] = conjx(x.e[b][a]);
-  return r;
-}
-__device__ __forceinline__ M3d m3_ah(const M3d& x) {
-  M3d r;
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) r.e[a][b] = 0.5 * (x.e[a][b] - conjx(x.e[b][a]));
-  return r;
-}
-
-__device__ __forceinline__ int64_t lex_shift(const Geom& g, int64_t site, int dir, int sgn) {
-  int c[4];
-  int64_t r = site;
-#pragma unroll
-  for (int d = 0; d < 4; ++d) {
-    c[d] = int(r % g.L[d]);
-    r /= g.L[d];
-  }
-  c[dir] = (c[dir] + sgn + g.L[dir]) % g.L[dir];
-  return c[0] + int64_t(g.L[0]) * (c[1] + int64_t(g.L[1]) * (c[2] + int64_t(g.L[2]) * c[3]));
-}
-
-// v(x) = Vup(x)^dag - Vdn(x)^dag (staples.cpp:596-597, 641-643)
-__device__ M3d leaves(const Geom& g, const double* raw, int64_t V, int64_t x, int mu, int nu) {
-  const int64_t xn = lex_shift(g, x, nu, 1), xm = lex_shift(g, x, mu, 1);
-  M3d up = m3_mul(m3_mul(m3_load(raw, V, x, nu), m3_load(raw, V, xn, mu)), m3_dag(m3_load(raw, V, xm, nu)));
-  const int64_t y = lex_shift(g, x, nu, -1), ym = lex_shift(g, y, mu, 1);
-  M3d dn = m3_mul(m3_mul(m3_dag(m3_load(raw, V, y, nu)), m3_load(raw, V, y, mu)), m3_load(raw, V, ym, nu));
-  M3d a = m3_dag(up), b = m3_dag(dn), v;
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) v.e[i][j] = a.e[i][j] - b.e[i][j];
-  return v;
-}
-
-// Staples::fieldStrength (lib/Measurements/GaugeM/staples.cpp:587-666)
-__device__ M3d field_strength_at(const Geom& g, const double* raw, int64_t V, int64_t x, int mu, int nu) {
-  const int64_t xm = lex_shift(g, x, mu, -1);
-  M3d f1 = m3_ah(m3_mul(m3_load(raw, V, x, mu), leaves(g, raw, V, x, mu, nu)));
-  M3d f2 = m3_ah(m3_mul(leaves(g, raw, V, xm, mu, nu), m3_load(raw, V, xm, mu)));
-  M3d f;
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) f.e[i][j] = f1.e[i][j] + f2.e[i][j];
-  // traceless anti-Hermitian part (anti_hermite_traceless, sunMatUtils.cpp:50-55), x 0.25
-  const double imtr = (f.e[0][0].im + f.e[1][1].im + f.e[2][2].im) / 3.0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) f.e[i][i].im -= imtr;
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) f.e[i][j] = 0.25 * f.e[i][j];
-  return f;
-}
-
-__global__ void field_strength_kernel(Geom g, const double* raw, int mu, int nu, double* out) {
-  const int64_t V = 2 * int64_t(g.Vh);
-  for (int64_t x = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < V;
-       x += int64_t(gridDim.x) * blockDim.x) {
-    M3d f = field_strength_at(g, raw, V, x, mu, nu);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        out[18 * x + 2 * (3 * i + j)] = f.e[i][j].re;
-        out[18 * x + 2 * (3 * i + j) + 1] = f.e[i][j].im;
-      }
-  }
-}
-
-cudaError_t launch_field_strength(const Geom& g, const double* raw, int mu, int nu, double* out,
-                                  cudaStream_t st) {
-  field_strength_kernel<<<grid_for(2 * int64_t(g.Vh), 128), 128, 0, st>>>(g, raw, mu, nu, out);
-  return cudaGetLastError();
-}
-
-// complex 6x6 inverse by Gauss-Jordan elimination with partial pivoting
-__device__ bool inv6(Cx<double> a[6][6], Cx<double> inv[6][6]) {
-  for (int i = 0; i < 6; ++i)
-    for (int j = 0; j < 6; ++j) inv[i][j] = {i == j ? 1.0 : 0.0, 0.0};
-  for (int c = 0; c < 6; ++c) {
-    int piv = c;
-    double best = a[c][c].re * a[c][c].re + a[c][c].im * a[c][c].im;
-    for (int r = c + 1; r < 6; ++r) {
-      const double m = a[r][c].re * a[r][c].re + a[r][c].im * a[r][c].im;
-      if (m > best) {
-        best = m;
-        piv = r;
-      }
-    }
-    if (!(best > 0.0)) return false;
-    if (piv != c)
-      for (int j = 0; j < 6; ++j) {
-        Cx<double> t = a[c][j]; a[c][j] = a[piv][j]; a[piv][j] = t;
-        t = inv[c][j]; inv[c][j] = inv[piv][j]; inv[piv][j] = t;
-      }
-    const double den = a[c][c].re * a[c][c].re + a[c][c].im * a[c][c].im;
-    const Cx<double> rp = {a[c][c].re / den, -a[c][c].im / den};
-    for (int j = 0; j < 6; ++j) {
-      a[c][j] = a[c][j] * rp;
-      inv[c][j] = inv[c][j] * rp;
-    }
-    for (int r = 0; r < 6; ++r) {
-      if (r == c) continue;
-      const Cx<double> f = a[r][c];
-      for (int j = 0; j < 6; ++j) {
-        a[r][j] = a[r][j] - f * a[c][j];
-        inv[r][j] = inv[r][j] - f * inv[c][j];
-      }
-    }
-  }
-  return true;
-}
-
-__device__ void store_block(const CloverArrays& ca, bool inverse, int p, int64_t Vh, int64_t hs,
-                            int blk, Cx<double> m[6][6]) {
-  // Hermitian parts: real diagonal and upper triangle (averaged with the lower)
-  double v[36];
-  for (int i = 0; i < 6; ++i) v[i] = m[i][i].re;
-  for (int i = 0; i < 6; ++i)
-    for (int j = i + 1; j < 6; ++j) {
-      const int k = tri(i, j);
-      v[6 + 2 * k] = 0.5 * (m[i][j].re + m[j][i].re);
-      v[7 + 2 * k] = 0.5 * (m[i][j].im - m[j][i].im);
-    }
-  void* const* arr = inverse ? ca.Ainv[0] : ca.A[0];
-  double2* d = static_cast<double2*>(arr[p]);
-  for (int k = 0; k < 18; ++k) d[blk0<36>(hs) + 32 * (blk * 18 + k)] = make_double2(v[2 * k], v[2 * k + 1]);
-  float* fptr = reinterpret_cast<float*>(static_cast<float4*>((inverse ? ca.Ainv[1] : ca.A[1])[p]));
-  // FP32: 18 float4 chunks over both blocks, values v_all[36*blk + j]
-  for (int q = 0; q < 9; ++q) {
-    float4 f4 = make_float4(float(v[4 * q]), float(v[4 * q + 1]), float(v[4 * q + 2]), float(v[4 * q + 3]));
-    reinterpret_cast<float4*>(fptr)[blk0<18>(hs) + 32 * (blk * 9 + q)] = f4;
-  }
-  uint4* h = static_cast<uint4*>((inverse ? ca.Ainv[2] : ca.A[2])[p]);
-  // FP16: 9 chunks of 8 halves over both blocks: block 0 owns values 0..35,
-  // block 1 36..71; chunk 4 straddles the two blocks (values 32..39).
-  // Written per half-word pair so the two blocks can be stored independently.
-  unsigned short* hs16 = reinterpret_cast<unsigned short*>(h);
-  for (int j = 0; j < 36; ++j) {
-    const int gidx = 36 * blk + j;
-    const int q = gidx / 8, w = gidx % 8;
-    __half hv = __float2half_rn(float(v[j]));
-    hs16[(blk0<9>(hs) + 32 * q) * 8 + w] = *reinterpret_cast<unsigned short*>(&hv);
-  }
-}
-
-__global__ void clover_build_kernel(Geom g, const double* raw, double kc, CloverArrays ca, int* singular) {
-  const int64_t Vh = g.Vh;
-  const int64_t V = 2 * Vh;
-  const int PAIRS[6][2] = {{1, 2}, {2, 0}, {0, 1}, {3, 0}, {3, 1}, {3, 2}};
-  for (int64_t x = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < V;
-       x += int64_t(gridDim.x) * blockDim.x) {
-    int c4[4];
-    int64_t rr = x;
-    for (int d = 0; d < 4; ++d) {
-      c4[d] = int(rr % g.L[d]);
-      rr /= g.L[d];
-    }
-    const int p = (c4[0] + c4[1] + c4[2] + c4[3]) & 1;
-    const int64_t hs = x >> 1;
-    Cx<double> B[2][6][6];
-    for (int s = 0; s < 2; ++s)
-      for (int i = 0; i < 6; ++i)
-        for (int j = 0; j < 6; ++j) B[s][i][j] = {i == j ? 1.0 : 0.0, 0.0};
-    for (int k = 0; k < 6; ++k) {
-      const M3d F = field_strength_at(g, raw, V, x, PAIRS[k][0], PAIRS[k][1]);
-      for (int s = 0; s < 2; ++s)
-        for (int a = 0; a < 2; ++a)
-          for (int b = 0; b < 2; ++b) {
-            const double2 sv = c_spm[s][k][a][b];
-            if (sv.x == 0.0 && sv.y == 0.0) continue;
-            const Cx<double> sc = {-kc * sv.x, -kc * sv.y};
-            for (int i = 0; i < 3; ++i)
-              for (int j = 0; j < 3; ++j) B[s][a * 3 + i][b * 3 + j] = B[s][a * 3 + i][b * 3 + j] + sc * F.e[i][j];
-          }
-    }
-    for (int s = 0; s < 2; ++s) {
-      Cx<double> inv[6][6], work[6][6];
-      for (int i = 0; i < 6; ++i)
-        for (int j = 0; j < 6; ++j) work[i][j] = B[s][i][j];
-      if (!inv6(work, inv)) atomicExch(singular, 1);
-      store_block(ca, false, p, Vh, hs, s, B[s]);
-      store_block(ca, true, p, Vh, hs, s, inv);
-    }
-  }
-}
-
-cudaError_t launch_clover_build(const Geom& g, const double* raw, double kappa_csw,
-                                CloverArrays ca, int* singular, cudaStream_t st) {
-  clover_build_kernel<<<grid_for(2 * int64_t(g.Vh), 64), 64, 0, st>>>(g, raw, kappa_csw, ca, singular);
-  return cudaGetLastError();
-}
-
-void clover_init_tables() {
-  // S_k[s_out][s_in] as (re, im), from Dirac_Clover::isigma_* (dirac_clover.cpp:221-329)
-  double S[6][4][4][2];
-  std::memset(S, 0, sizeof(S));
-  auto set = [&](int k, int a, int b, double re, double im) {
-    S[k][a][b][0] = re;
-    S[k][a][b][1] = im;
-  };
-  // isigma_23: w0 = i v1, w1 = i v0, w2 = i v3, w3 = i v2
-  set(0, 0, 1, 0, 1); set(0, 1, 0, 0, 1); set(0, 2, 3, 0, 1); set(0, 3, 2, 0, 1);
-  // isigma_31: w0 = v1, w1 = -v0, w2 = v3, w3 = -v2
-  set(1, 0, 1, 1, 0); set(1, 1, 0, -1, 0); set(1, 2, 3, 1, 0); set(1, 3, 2, -1, 0);
-  // isigma_12: w0 = i v0, w1 = -i v1, w2 = i v2, w3 = -i v3
-  set(2, 0, 0, 0, 1); set(2, 1, 1, 0, -1); set(2, 2, 2, 0, 1); set(2, 3, 3, 0, -1);
-  // isigma_41: w0 = -i v3, w1 = -i v2, w2 = -i v1, w3 = -i v0
-  set(3, 0, 3, 0, -1); set(3, 1, 2, 0, -1); set(3, 2, 1, 0, -1); set(3, 3, 0, 0, -1);
-  // isigma_42: w0 = -v3, w1 = v2, w2 = -v1, w3 = v0
-  set(4, 0, 3, -1, 0); set(4, 1, 2, 1, 0); set(4, 2, 1, -1, 0); set(4, 3, 0, 1, 0);
-  // isigma_43: w0 = -i v2, w1 = i v3, w2 = -i v0, w3 = i v1
-  set(5, 0, 2, 0, -1); set(5, 1, 3, 0, 1); set(5, 2, 0, 0, -1); set(5, 3, 1, 0, 1);
-  double2 spm[2][6][2][2];
-  for (int s = 0; s < 2; ++s)
-    for (int k = 0; k < 6; ++k)
-      for (int a = 0; a < 2; ++a)
-        for (int b = 0; b < 2; ++b) {
-          const double sg = s == 0 ? 1.0 : -1.0;
-          spm[s][k][a][b].x = S[k][a][b][0] + sg * S[k][a][b + 2][0];
-          spm[s][k][a][b].y = S[k][a][b][1] + sg * S[k][a][b + 2][1];
-        }
-  cudaMemcpyToSymbol(c_spm, spm, sizeof(spm));
-}
-
-}  // namespace iro
-
-namespace iro {
-
 // ---- mixed-precision reliable updates -------------------------------------------------
 // The blocks are multiples of nrhs (launch_cfg), so a thread keeps one
 // right-hand side across its grid-stride loop.

@@ -49,7 +49,7 @@ int clover_ready(iro_ctx* c, double mass, double csw);
 CloverPtr clover(iro_ctx* c, int prec, int p, bool inverse);
 GaugePtr gauge_double(iro_ctx* c);
 int gauge_recon(iro_ctx* c);
-const double* gauge_format_g(iro_ctx* c);
+const double2* gauge_d18(iro_ctx* c);
 bool gauge_loaded(iro_ctx* c);
 const Geom& geom(iro_ctx* c);
 int64_t volume(iro_ctx* c);
@@ -1164,7 +1164,7 @@ extern "C" int iro_md_force(iro_ctx* c, int op, double mass, double csw, const d
   // the force and (clover) Lambda_k in the context's solver scratch, which
   // stays allocated: repeated calls allocate nothing
   const size_t f_bytes = (nF * sizeof(double) + 255) / 256 * 256;
-  char* scr = static_cast<char*>(scratch(c, f_bytes + nL * sizeof(double2), &rc));
+  char* scr = static_cast<char*>(scratch(c, f_bytes + nL * sizeof(double), &rc));
   if (!scr) return rc;
   double* F = reinterpret_cast<double*>(scr);
   CK(cudaMemsetAsync(F, 0, nF * sizeof(double), st));
@@ -1178,12 +1178,12 @@ extern "C" int iro_md_force(iro_ctx* c, int op, double mass, double csw, const d
     }
     if (clover_term) {
       // the clover block of Dirac_Clover::md_force: Lambda_k for the 6 planes
-      // (6 * 9 complex per site), then the leaf derivatives; its site offsets
-      // reach two sites out, which one periodic wrap covers for extents >= 2
+      // (6 * 9 reals per site), then the derivatives of the plaquettes through
+      // each link
       for (int d = 0; d < 4; ++d)
         if (g.L[d] < 2) return set_error(c, IRO_BAD_ARG, "clover force needs every extent >= 2");
-      double2* lam = reinterpret_cast<double2*>(scr + f_bytes);
-      CK(launch_clover_force(g, gauge_format_g(c), E->half(0), E->half(1), Z->half(0), Z->half(1),
+      double* lam = reinterpret_cast<double*>(scr + f_bytes);
+      CK(launch_clover_force(g, gauge_d18(c), E->half(0), E->half(1), Z->half(0), Z->half(1),
                              -k * csw / 4.0, lam, F, st));
     }
   } else {
