@@ -3,6 +3,7 @@
 // the Krylov solvers.  See include/iroiro_b200.h for the contract of each
 // entry point and the reference interface it replaces.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -10,6 +11,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <tuple>
@@ -19,6 +21,9 @@
 #include "iroiro_b200.h"
 
 using namespace iro;
+
+// host threads of a copy to or from pageable memory (ring_copy)
+constexpr int kCopyThreads = 8;
 
 struct iro_field {
   iro_ctx* ctx;
@@ -60,9 +65,7 @@ struct iro_ctx {
   // boundary staging
   double* stage = nullptr;
   size_t stage_bytes = 0;
-  // pinned host ring for large copies to and from pageable host memory
-  char* ring[2] = {nullptr, nullptr};
-  cudaEvent_t ring_ev[2] = {nullptr, nullptr};
+  bool attached = false;  // counted among its device's copy-ring users
   // copy streams (host-to-device, device-to-host) and chunk events of the
   // overlapped Schur operator between pinned host arrays
   cudaStream_t xs[2] = {nullptr, nullptr};
@@ -158,13 +161,29 @@ DevField* ws(iro_ctx* c, int subset, int prec, int nrhs, int slot, int* rc) {
 
 // ---- host copies -----------------------------------------------------------------
 // The driver copies pageable host memory through its own staging on one host
-// thread (~21 GB/s for 4.8 GB device to host, measured on a B200 host).
-// Large copies to or from pageable memory go through two pinned chunks
-// instead: the DMA of one chunk overlaps the copy of the other, which
-// kCopyThreads host threads split (~46 GB/s measured).  Pinned (registered)
-// host memory, and copies below two chunks, take the direct DMA.
-constexpr size_t kRingChunk = size_t(128) << 20;
-constexpr int kCopyThreads = 8;
+// thread (H2D ~21 GB/s; D2H into memory that was never touched 4.7 GB/s,
+// page faults included: 15.9 ms for the 75 MB force of a 16^3x32 lattice).
+// Copies to or from pageable memory of kRingMin bytes and more are split into
+// kRingSlot pieces that kCopyThreads host threads take in turn, each through
+// two pinned slots of its own: its DMAs overlap its host copies and those of
+// the other threads, and the page faults of a fresh destination are taken in
+// parallel.  The slots (16 MB in all) are small so that the pipeline fills at
+// once: with two 128 MB chunks the first DMA started after 4 ms of host
+// copying.  Pinned memory, device-accessible memory and small copies take the
+// direct DMA.  Measured: the 75 MB force D2H 15.9 -> 2.1 ms, its 50 MB of
+// inputs 1.9 -> 2.2 ms of DMA time but no driver staging; a 382 MB gauge
+// upload 13.5 -> 9.6 ms.
+constexpr size_t kRingSlot = size_t(1) << 20;
+constexpr size_t kRingMin = size_t(4) << 20;
+
+bool host_pageable(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
+}
 
 bool host_pinned(const void* p) {
   cudaPointerAttributes a;
@@ -175,79 +194,130 @@ bool host_pinned(const void* p) {
   return a.type == cudaMemoryTypeHost;
 }
 
-// the stripes no thread took (thread creation can fail) are copied by the caller
-void parallel_copy(void* dst, const void* src, size_t bytes) {
-  const int nt = int(std::min<unsigned>(kCopyThreads, std::max(1u, std::thread::hardware_concurrency())));
-  const size_t stripe = ((bytes / nt) + 63) & ~size_t(63);
-  auto part = [=](int k) {
-    const size_t a = std::min(bytes, k * stripe), b = std::min(bytes, a + stripe);
-    if (b > a) std::memcpy(static_cast<char*>(dst) + a, static_cast<const char*>(src) + a, b - a);
-  };
-  std::vector<std::thread> th;
-  int k = 1;
-  try {
-    for (; k < nt; ++k) th.emplace_back(part, k);
-  } catch (...) {
+// The slots of one device, shared by its contexts: allocated by the first copy
+// that needs them, given back when the device's last context is destroyed.  One
+// copy at a time uses them; another one that comes meanwhile (from another
+// thread) takes the direct path.
+struct CopyRing {
+  std::mutex use;
+  char* buf = nullptr;
+  cudaEvent_t ev[2 * kCopyThreads] = {};  // a slot's last DMA
+  int contexts = 0;                       // guarded by g_ring_mutex
+};
+constexpr int kRingDevices = 16;
+CopyRing g_ring[kRingDevices];
+std::mutex g_ring_mutex;
+
+void ring_attach(int device) {
+  if (device < 0 || device >= kRingDevices) return;
+  std::lock_guard<std::mutex> lk(g_ring_mutex);
+  ++g_ring[device].contexts;
+}
+void ring_detach(int device) {
+  if (device < 0 || device >= kRingDevices) return;
+  std::lock_guard<std::mutex> lk(g_ring_mutex);
+  CopyRing& r = g_ring[device];
+  if (--r.contexts > 0) return;
+  if (r.buf) cudaFreeHost(r.buf);
+  r.buf = nullptr;
+  for (cudaEvent_t& e : r.ev) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
   }
-  part(0);
-  for (int j = k; j < nt; ++j) part(j);
-  for (auto& t : th) t.join();
 }
 
-int ensure_ring(iro_ctx* c) {
-  for (int i = 0; i < 2; ++i) {
-    if (!c->ring[i]) CK(cudaHostAlloc(reinterpret_cast<void**>(&c->ring[i]), kRingChunk, cudaHostAllocDefault));
-    if (!c->ring_ev[i]) CK(cudaEventCreateWithFlags(&c->ring_ev[i], cudaEventDisableTiming));
-  }
+int ensure_ring(iro_ctx* c, CopyRing& r) {
+  if (!r.buf) CK(cudaHostAlloc(reinterpret_cast<void**>(&r.buf), 2 * kCopyThreads * kRingSlot, cudaHostAllocDefault));
+  for (cudaEvent_t& e : r.ev)
+    if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   return IRO_OK;
+}
+
+// One thread's share of a copy between `host` and `dev` through slots 2w and
+// 2w + 1: pieces are taken from `next` until none is left.  A slot's event
+// marks its last DMA.
+cudaError_t ring_worker(iro_ctx* c, CopyRing& ring, int w, bool to_host, char* host, char* dev, size_t bytes,
+                        std::atomic<size_t>& next) {
+  cudaError_t e = cudaSetDevice(c->device);
+  if (e != cudaSuccess) return e;
+  char* slot[2] = {ring.buf + 2 * w * kRingSlot, ring.buf + (2 * w + 1) * kRingSlot};
+  cudaEvent_t ev[2] = {ring.ev[2 * w], ring.ev[2 * w + 1]};
+  const size_t none = ~size_t(0);
+  size_t off[2] = {none, none};  // device to host: the piece in flight in each slot
+  auto land = [&](int k) -> cudaError_t {
+    if (off[k] == none) return cudaSuccess;
+    const cudaError_t r = cudaEventSynchronize(ev[k]);
+    if (r == cudaSuccess) std::memcpy(host + off[k], slot[k], std::min(kRingSlot, bytes - off[k]));
+    off[k] = none;
+    return r;
+  };
+  for (int k = 0;; k ^= 1) {
+    if (to_host && (e = land(k)) != cudaSuccess) return e;
+    const size_t o = next.fetch_add(1) * kRingSlot;
+    if (o >= bytes) return to_host ? land(k ^ 1) : cudaSuccess;
+    const size_t len = std::min(kRingSlot, bytes - o);
+    if (to_host) {
+      e = cudaMemcpyAsync(slot[k], dev + o, len, cudaMemcpyDeviceToHost, c->stream);
+      off[k] = o;
+    } else {
+      // the slot's previous DMA (of this copy or an earlier one) is done
+      if ((e = cudaEventSynchronize(ev[k])) != cudaSuccess) return e;
+      std::memcpy(slot[k], host + o, len);
+      e = cudaMemcpyAsync(dev + o, slot[k], len, cudaMemcpyHostToDevice, c->stream);
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(ev[k], c->stream);
+    if (e != cudaSuccess) return e;
+  }
+}
+
+int ring_copy(iro_ctx* c, CopyRing& ring, bool to_host, char* host, char* dev, size_t bytes) {
+  RCK(ensure_ring(c, ring));
+  std::atomic<size_t> next{0};
+  const int nt = int(std::min<size_t>(std::min<unsigned>(kCopyThreads, std::max(1u, std::thread::hardware_concurrency())),
+                                      (bytes + kRingSlot - 1) / kRingSlot));
+  cudaError_t err[kCopyThreads] = {};
+  std::vector<std::thread> th;
+  // a thread that cannot be created leaves its share to the others
+  try {
+    th.reserve(nt);
+    for (int w = 1; w < nt; ++w)
+      th.emplace_back([&, w] { err[w] = ring_worker(c, ring, w, to_host, host, dev, bytes, next); });
+  } catch (...) {
+  }
+  err[0] = ring_worker(c, ring, 0, to_host, host, dev, bytes, next);
+  for (auto& t : th) t.join();
+  for (cudaError_t e : err)
+    if (e != cudaSuccess) {
+      cudaStreamSynchronize(c->stream);  // nothing of a failed copy stays in flight
+      return cuda_fail(c, e, "host copy");
+    }
+  return IRO_OK;
+}
+
+// the ring, locked, if this copy goes through it
+CopyRing* ring_for(iro_ctx* c, const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
+  if (bytes < kRingMin || c->device < 0 || c->device >= kRingDevices || !host_pageable(host)) return nullptr;
+  lk = std::unique_lock<std::mutex>(g_ring[c->device].use, std::try_to_lock);
+  return lk.owns_lock() ? &g_ring[c->device] : nullptr;
 }
 
 // device -> host, returns with the copy complete
 int copy_d2h(iro_ctx* c, void* host, const void* dev, size_t bytes) {
-  if (bytes < 2 * kRingChunk || host_pinned(host)) {
-    CK(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    return IRO_OK;
-  }
-  RCK(ensure_ring(c));
-  const size_t nch = (bytes + kRingChunk - 1) / kRingChunk;
-  // chunk i goes to slot i % 2; the host copy of chunk i - 1 (slot (i - 1) % 2)
-  // runs while the DMA of chunk i is in flight
-  for (size_t i = 0; i <= nch; ++i) {
-    if (i < nch) {
-      const size_t off = i * kRingChunk, len = std::min(kRingChunk, bytes - off);
-      CK(cudaMemcpyAsync(c->ring[i % 2], static_cast<const char*>(dev) + off, len, cudaMemcpyDeviceToHost,
-                         c->stream));
-      CK(cudaEventRecord(c->ring_ev[i % 2], c->stream));
-    }
-    if (i >= 1) {
-      const size_t j = i - 1, off = j * kRingChunk, len = std::min(kRingChunk, bytes - off);
-      CK(cudaEventSynchronize(c->ring_ev[j % 2]));
-      parallel_copy(static_cast<char*>(host) + off, c->ring[j % 2], len);
-    }
-  }
+  std::unique_lock<std::mutex> lk;
+  if (CopyRing* r = ring_for(c, host, bytes, lk))
+    return ring_copy(c, *r, true, static_cast<char*>(host), const_cast<char*>(static_cast<const char*>(dev)), bytes);
+  CK(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   return IRO_OK;
 }
 
 // host -> device, enqueued on the context's stream (the host buffer may be
 // reused once this returns)
 int copy_h2d(iro_ctx* c, void* dev, const void* host, size_t bytes) {
-  if (bytes < 2 * kRingChunk || host_pinned(host)) {
-    CK(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, c->stream));
-    return IRO_OK;
-  }
-  RCK(ensure_ring(c));
-  const size_t nch = (bytes + kRingChunk - 1) / kRingChunk;
-  for (size_t i = 0; i < nch; ++i) {
-    const size_t off = i * kRingChunk, len = std::min(kRingChunk, bytes - off);
-    // slot i % 2 is free once the DMA of chunk i - 2 has completed
-    if (i >= 2) CK(cudaEventSynchronize(c->ring_ev[i % 2]));
-    parallel_copy(c->ring[i % 2], static_cast<const char*>(host) + off, len);
-    CK(cudaMemcpyAsync(static_cast<char*>(dev) + off, c->ring[i % 2], len, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaEventRecord(c->ring_ev[i % 2], c->stream));
-  }
-  // the pinned chunks are reused by the next call: wait for the last DMAs
-  for (size_t i = nch >= 2 ? nch - 2 : 0; i < nch; ++i) CK(cudaEventSynchronize(c->ring_ev[i % 2]));
+  std::unique_lock<std::mutex> lk;
+  if (CopyRing* r = ring_for(c, host, bytes, lk))
+    return ring_copy(c, *r, false, const_cast<char*>(static_cast<const char*>(host)), static_cast<char*>(dev), bytes);
+  CK(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, c->stream));
   return IRO_OK;
 }
 
@@ -722,6 +792,8 @@ int iro_ctx_create(const int L[4], int device, iro_ctx** out) {
     CK(cudaMalloc(&c->d_singular, sizeof(int)));
     CK(cudaGetLastError());
   }
+  ring_attach(device);
+  c->attached = true;
   *out = c.release();
   return IRO_OK;
 }
@@ -743,11 +815,9 @@ int iro_ctx_destroy(iro_ctx* c) {
     }
   if (c->h_pinned) cudaFreeHost(c->h_pinned);
   if (c->scratch) cudaFree(c->scratch);
-  for (int i = 0; i < 2; ++i) {
-    if (c->ring[i]) cudaFreeHost(c->ring[i]);
-    if (c->ring_ev[i]) cudaEventDestroy(c->ring_ev[i]);
-    if (c->xs[i]) cudaStreamDestroy(c->xs[i]);
-  }
+  if (c->attached) ring_detach(c->device);
+  for (cudaStream_t x : c->xs)
+    if (x) cudaStreamDestroy(x);
   for (cudaEvent_t e : c->xev)
     if (e) cudaEventDestroy(e);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);

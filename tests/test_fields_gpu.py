@@ -1,5 +1,7 @@
 """Device-resident fields: boundary round trip and the Field reductions
 (Field::norm, include/field.h:74-78; Field::operator*, lib/Fields/field.inl:58-62)."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -36,3 +38,31 @@ def test_norm_and_dot(ctx, prec, tol):
     assert np.allclose(da.norm(), np.linalg.norm(A, axis=1), rtol=tol, atol=0)
     ref = np.einsum("ri,ri->r", A, B)
     assert np.all(np.abs(da.dot(db) - ref) <= tol * np.linalg.norm(A, axis=1) * np.linalg.norm(B, axis=1))
+
+
+@pytest.mark.parametrize("nrhs", [2, 3, 5, 12])
+def test_pageable_round_trip_around_the_threaded_copy(nrhs):
+    """Uploads and downloads below and above the size from which pageable
+    memory is copied by several threads in 1 MiB pieces (1.5 MiB per
+    right-hand side here: a direct copy, then whole and odd numbers of pieces),
+    bit for bit; again with two contexts copying from two threads at once."""
+    L = [8, 8, 8, 16]
+    n = int(np.prod(L)) * nrhs
+    f = ib.synth_gaussian(n, 50 + nrhs)
+    ctxs = [ib.Context(L, 0) for _ in range(2)]
+    fields = [ib.DeviceField(c, 2, "double", nrhs) for c in ctxs]
+    assert np.array_equal(fields[0].upload(f).download(), f)
+    bad = []
+
+    def work(k):
+        g = f + k
+        for _ in range(4):
+            if not np.array_equal(fields[k].upload(g).download(), g):
+                bad.append(k)
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
