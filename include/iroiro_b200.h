@@ -370,10 +370,10 @@ int iro_gcr_solve_field(iro_ctx* ctx, int op, double mass, double csw, const iro
                         iro_gcr_out* out);
 
 /* Self-test of the device-side bounded waits (no counterpart in the
-   reference): the tensor-core kernels wait on mbarriers for at most 1 s and
-   then set an error flag that the host turns into IRO_TIMEOUT, leaving the
-   context usable.  This runs the same wait on an mbarrier that nothing
-   arrives at, for limit_ms (0 < limit_ms <= 1000), and returns IRO_TIMEOUT
+   reference): a kernel that waits (the small-lattice CG's grid barrier) does so
+   for at most 1 s and then sets an error flag that the host turns into
+   IRO_TIMEOUT, leaving the context usable.  This runs such a wait on an mbarrier
+   that nothing arrives at, for limit_ms (0 < limit_ms <= 1000), and returns IRO_TIMEOUT
    with the time it waited in *waited_ms. */
 int iro_selftest_bounded_wait(iro_ctx* ctx, double limit_ms, double* waited_ms);
 

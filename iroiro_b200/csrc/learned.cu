@@ -12,18 +12,17 @@
 // parallel-transport convolutions of Lehner & Wettig, "Gauge-equivariant
 // neural networks as preconditioners in lattice QCD", PRD 108 (2023).
 //
-// Forward kernel, tiles of 32 sites = 96 rows (site, colour):
-//  1. the CUDA cores transport every input channel along the 9 displacements
-//     and write the real GEMM operand A[row][k], k = (2d + re/im)*C_in + i,
-//     in BF16 into shared memory in the canonical K-major no-swizzle UMMA
-//     layout (8x16-byte core matrices);
-//  2. one thread issues tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M=128)
-//     against the packed real weight matrix B[n][k] (n = 2*o + re/im), the
-//     accumulator lives in tensor memory;
-//  3. three warps read their 32 accumulator lanes back (tcgen05.ld) and
-//     store the output channels in FP32.
-// Every wait on the MMA's mbarrier is bounded: on time-out the kernel sets
-// an error flag, skips the read-back, frees its tensor memory and returns.
+// Forward kernel: every warp works alone on tiles of 32 sites = 96 rows (site,
+// colour).  Per displacement it transports the input channels on the CUDA
+// cores (lane = site), stages them as BF16 rows in shared memory and multiplies
+// them with the displacement's weights on the tensor cores (mma.sync, BF16 x
+// BF16 -> FP32, the accumulators in registers over all nine displacements),
+// then stores the output channels in FP32.  The contraction is small (K = 8 or
+// 16 per displacement and a few output columns): what bounds a layer is the
+// latency of the gathers.  A block-wide version, nine warps building one
+// operand for tcgen05.mma in tensor memory, spent its time at the block's
+// barriers: (4,4,4,4) at 32^3x64 1.30 ms, 0.95 ms now; (4,16,16,16,4) at
+// 24^3x48 1.74 and 1.31 ms.
 //
 // Backward: the gradient of the input is a layer of the same kind on dY, with
 // adjoint weights and the displacements reversed (T_{+mu}^dag = T_{-mu}), so it
@@ -42,28 +41,9 @@
 
 namespace iro {
 
-// ---- tcgen05 / mbarrier primitives ------------------------------------------------
+// ---- shared-memory addresses; the bounded mbarrier wait of the self-test -----------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
-               "r"(ncols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void fence_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -81,11 +61,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t phase) {
   return ok != 0;
 }
 
-// A wait on an mbarrier gives up after kWaitNs nanoseconds of global time
-// (or kWaitLimit polls, whichever comes first): the kernel then sets its
-// error flag and leaves, and the host reports IRO_TIMEOUT.
+// A wait on an mbarrier gives up after a limit of global time (or kWaitLimit
+// polls, whichever comes first): the kernel then sets its error flag and
+// leaves, and the host reports IRO_TIMEOUT.
 constexpr int kWaitLimit = 1 << 24;
-constexpr uint64_t kWaitNs = 1000000000ull;
 
 __device__ __forceinline__ uint64_t global_ns() {
   uint64_t t;
@@ -95,8 +74,7 @@ __device__ __forceinline__ uint64_t global_ns() {
 
 // Polls the barrier until `phase` completes; false after limit_ns of global
 // time or kWaitLimit polls
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t phase,
-                                                  uint64_t limit_ns = kWaitNs) {
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t phase, uint64_t limit_ns) {
   const uint64_t t0 = global_ns();
   for (int it = 0; it < kWaitLimit; ++it) {
     if (mbar_try_wait(bar, phase)) return true;
@@ -104,66 +82,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t phase,
   }
   return false;
 }
-// D(tmem) (+)= A(smem) * B(smem)^T, BF16 inputs, FP32 accumulation
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(bar))
-      : "memory");
-}
-// 16 consecutive FP32 accumulator columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
-}
 
-// Shared-memory matrix descriptor, K-major, no swizzle: 8-row x 16-byte core
-// matrices, LBO = byte step between the two K-halves of an MMA's K=16, SBO =
-// byte step between 8-row groups; version 1 (sm100).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  return uint64_t((addr >> 4) & 0x3FFFu) | (uint64_t((lbo >> 4) & 0x3FFFu) << 16) |
-         (uint64_t((sbo >> 4) & 0x3FFFu) << 32) | (uint64_t(1) << 46);
-}
-// Instruction descriptor: FP32 accumulate, BF16 A and B, both K-major, M=128, N.
-__host__ __device__ constexpr uint32_t idesc_bf16(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(128 >> 4) << 24);
-}
-// byte offset of element (r, k) of a K-major R x K BF16 operand in the canonical layout
-__host__ __device__ __forceinline__ uint32_t canon(int r, int k, int K) {
-  return uint32_t((r >> 3) * (K / 8) * 128 + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
-}
-
+// K and N of the packed real weights B[n][k]: k = (2d + re/im) CIN + i, n = 2o +
+// re/im, padded to multiples of 16
 template <int CIN, int COUT>
 struct Ptc {
   static constexpr int KF = 18 * CIN;
   static constexpr int KP = (KF + 15) / 16 * 16;
-  static constexpr int NF = 2 * COUT;
-  static constexpr int NP = NF < 16 ? 16 : (NF + 15) / 16 * 16;
-  static constexpr int TCOLS = NP <= 32 ? 32 : 64;
-  static constexpr int B_BYTES = NP * KP * 2;
-  // forward kernel: A holds the 96 rows of 32 sites; the MMA's rows 96..127
-  // read the bytes that follow (the weights, padded to at least 32 rows),
-  // which only feed accumulator rows that are never read back
-  static constexpr int A96_BYTES = 96 * KP * 2;
-  static constexpr int BF_BYTES = NP >= 32 ? B_BYTES : 32 * KP * 2;
 };
 
 // Feature element (site s, channel o, colour a) of a V-site field.  Channels
@@ -189,44 +114,8 @@ struct PtcGeo {
   Geom g;
   GaugePtr gauge;  // FP32 two-row links
   int V;
-  int* err;
   const int* skip;  // forward only: when set and nonzero the launch does nothing
 };
-
-// Issues the K/16 MMAs of D = A B^T into TMEM, commits to the mbarrier and
-// waits (bounded).  Only warp 0 polls the barrier (the other warps wait at
-// the block barrier without taking issue slots); the block barrier then
-// orders everyone's tcgen05 accesses after the completed MMAs.  Returns false
-// on time-out, in every thread.
-template <int K>
-__device__ bool mma_and_wait(const unsigned char* A, const unsigned char* B, uint32_t tmem,
-                             uint32_t idesc, uint64_t* bar, uint32_t phase, int* err) {
-  __shared__ int mma_ok;
-  fence_async_smem();
-  __syncthreads();
-  tc_fence_after();
-  if (threadIdx.x < 32) {
-    if (threadIdx.x == 0) {
-      const uint32_t a0 = smem_u32(A), b0 = smem_u32(B);
-      constexpr uint32_t sbo = (K / 8) * 128;
-#pragma unroll 1
-      for (int kb = 0; kb < K / 16; ++kb)
-        umma_bf16(tmem, smem_desc(a0 + kb * 256, 128, sbo), smem_desc(b0 + kb * 256, 128, sbo),
-                  idesc, kb > 0 ? 1u : 0u);
-      umma_commit(bar);
-    }
-    __syncwarp();
-    const bool ok = mbar_wait_bounded(bar, phase);
-    if (threadIdx.x == 0) {
-      mma_ok = ok ? 1 : 0;
-      if (!ok && err) atomicExch(err, 1);
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  return mma_ok != 0;
-}
 
 // ---- forward ----------------------------------------------------------------------
 // The CIN channel vectors of site s transported along displacement d, as
@@ -292,51 +181,6 @@ __device__ __forceinline__ void transport_words(const PtcGeo& G, const float2* _
   }
 }
 
-// Writes the A-tile entries of one (site, displacement) job: the CIN
-// transported channel vectors of the tile's site sl, as BF16 in columns
-// (2d + re/im)*CIN + i of rows 3*sl + colour; each colour row receives CIN/8
-// 16-byte stores (8-byte stores for CIN = 4).
-template <int CIN, int KP>
-__device__ __forceinline__ void a_tile_job(const PtcGeo& G, const float2* __restrict__ in, int s,
-                                           int sl, int d, unsigned char* A) {
-  constexpr int NW = CIN / 2;  // BF16x2 words per colour and part
-  uint32_t wre[3][NW], wim[3][NW];
-  if (s < G.V) {
-    transport_words<CIN>(G, in, s, d, wre, wim);
-  } else {
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int q = 0; q < NW; ++q) wre[r][q] = wim[r][q] = 0u;
-  }
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    const int row = 3 * sl + r;
-#pragma unroll
-    for (int part = 0; part < 2; ++part) {
-      const uint32_t* w = part ? wim[r] : wre[r];
-      const int k0 = (2 * d + part) * CIN;
-      if constexpr (CIN == 4) {
-        *reinterpret_cast<uint2*>(A + canon(row, k0, KP)) = make_uint2(w[0], w[1]);
-      } else {
-#pragma unroll
-        for (int q = 0; q < NW; q += 4)
-          *reinterpret_cast<uint4*>(A + canon(row, k0 + 2 * q, KP)) =
-              make_uint4(w[q], w[q + 1], w[q + 2], w[q + 3]);
-      }
-    }
-  }
-}
-
-// Persistent forward kernel: each CTA allocates its tensor memory, loads the
-// weights and zeroes its A tile once, then loops over tiles of 32 sites
-// (96 of the 128 MMA rows).  The 9 warps build the A tile, warp d handling
-// displacement d for the 32 sites (lane = site): branches on the displacement
-// are warp-uniform, a warp's gathers are the neighbours of 32 consecutive
-// sites, and its 16-byte stores into the canonical layout hit 8 different
-// bank groups per 128 bytes.  One thread issues the MMAs; warps 0-2 read the
-// accumulator back.  The mbarrier phase alternates per tile; every wait is
-// bounded and a time-out stops the CTA with the error flag set.
 constexpr int kFwdSites = 32;
 
 // First site of forward tile `tile`: even and odd tiles alternate (tile 2k is
@@ -350,181 +194,7 @@ constexpr int kFwdSites = 32;
 __device__ __forceinline__ int fwd_tile_site0(const PtcGeo& G, int tile) {
   return (tile & 1) * G.g.Vh + (tile >> 1) * kFwdSites;
 }
-constexpr int kFwdThreads = 288;
-
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(kFwdThreads) ptc_fwd_kernel(PtcGeo G, const float2* __restrict__ in,
-                                                              float2* __restrict__ out,
-                                                              const __nv_bfloat16* __restrict__ bop,
-                                                              int ntiles) {
-  if (G.skip && *G.skip) return;  // the same value in every thread, before any allocation
-  using S = Ptc<CIN, COUT>;
-  extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char* A = smem;
-  unsigned char* B = smem + S::A96_BYTES;
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ uint32_t tslot;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) tmem_alloc(&tslot, S::TCOLS);
-  if (threadIdx.x == 0) mbar_init(&bar, 1);
-  // zero the weights' padding rows (read only as A rows 96..127), then the
-  // weights: NP x KP row-major BF16, copied in 16-byte pieces into the canonical layout
-  for (int b = S::B_BYTES + threadIdx.x * 16; b < S::BF_BYTES; b += kFwdThreads * 16)
-    *reinterpret_cast<uint4*>(B + b) = make_uint4(0, 0, 0, 0);
-  for (int idx = threadIdx.x; idx < S::NP * (S::KP / 8); idx += kFwdThreads) {
-    const int n = idx / (S::KP / 8), k0 = (idx - n * (S::KP / 8)) * 8;
-    *reinterpret_cast<uint4*>(B + canon(n, k0, S::KP)) =
-        __ldg(reinterpret_cast<const uint4*>(bop + size_t(n) * S::KP + k0));
-  }
-  // columns KF..KP are never written by a job
-  for (int b = threadIdx.x * 16; b < S::A96_BYTES; b += kFwdThreads * 16)
-    *reinterpret_cast<uint4*>(A + b) = make_uint4(0, 0, 0, 0);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tslot;
-  uint32_t phase = 0;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int site0 = fwd_tile_site0(G, tile);
-    a_tile_job<CIN, S::KP>(G, in, site0 + lane, lane, warp, A);
-    const bool ok = mma_and_wait<S::KP>(A, B, tmem, idesc_bf16(S::NP), &bar, phase, G.err);
-    phase ^= 1u;
-    if (__syncthreads_or(!ok)) break;  // all threads leave together on a time-out
-    if (warp < 3) {
-      const int r = warp * 32 + lane;
-      float v[S::NP];
-#pragma unroll
-      for (int c = 0; c < S::NP; c += 16) tmem_ld16(tmem + (uint32_t(warp * 32) << 16) + c, v + c);
-      const int sl = r / 3, a = r - sl * 3;
-      const int s = site0 + sl;
-      if (s < G.V) {
-        // channel pair (2q, 2q+1) of colour a: one 16-byte store
-        float4* o4 = reinterpret_cast<float4*>(out) + size_t(a) * G.V + s;
-#pragma unroll
-        for (int q = 0; q < COUT / 2; ++q)
-          o4[size_t(3 * q) * G.V] = make_float4(v[4 * q], v[4 * q + 2], v[4 * q + 1], v[4 * q + 3]);
-      }
-    }
-    // the accumulator is read and the MMA has consumed A before the next tile
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, S::TCOLS);
-}
-
-// Double-buffered forward kernel (two A tiles, two accumulators): the A tile
-// of tile t+1 is built while the MMAs of tile t run; then the MMAs of tile t+1
-// are issued and tile t is read back while they run.  A CTA's tile
-// otherwise spends about a third of its time waiting for its MMAs (measured
-// with clock64 at 32^3x64: 3.5k of 9.5k cycles for an 8->8 layer).  The
-// shared memory holds [A1 | A0 | weights]: the MMA's rows 96..127 of A1 read
-// the first rows of A0, those of A0 the weights (padded to >= 32 rows); those
-// rows feed accumulator rows that are never read back.
-template <int CIN, int COUT>
-// (register budget: 4 CTAs per SM for 4 input channels, 3 for 8 -- what the
-// shared memory allows -- instead of the 2 that 84 registers left for 8;
-// 2.7 % less time per (4,8,8,4) application at 32^3x64)
-__global__ void __launch_bounds__(kFwdThreads, (CIN <= 4 ? 4 : (CIN <= 8 ? 3 : 1))) ptc_fwd2_kernel(PtcGeo G, const float2* __restrict__ in,
-                                                               float2* __restrict__ out,
-                                                               const __nv_bfloat16* __restrict__ bop,
-                                                               int ntiles) {
-  if (G.skip && *G.skip) return;  // the same value in every thread, before any allocation
-  using S = Ptc<CIN, COUT>;
-  extern __shared__ __align__(1024) unsigned char smem[];
-  // A tile of buffer b: A0 = smem + A96, A1 = smem
-  auto abuf = [&](int b) { return smem + (b ? 0 : S::A96_BYTES); };
-  unsigned char* B = smem + 2 * S::A96_BYTES;
-  __shared__ __align__(8) uint64_t bar[2];
-  __shared__ uint32_t tslot;
-  __shared__ int mma_ok;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) tmem_alloc(&tslot, 2 * S::TCOLS);
-  if (threadIdx.x == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-  }
-  for (int b = S::B_BYTES + threadIdx.x * 16; b < S::BF_BYTES; b += kFwdThreads * 16)
-    *reinterpret_cast<uint4*>(B + b) = make_uint4(0, 0, 0, 0);
-  for (int idx = threadIdx.x; idx < S::NP * (S::KP / 8); idx += kFwdThreads) {
-    const int n = idx / (S::KP / 8), k0 = (idx - n * (S::KP / 8)) * 8;
-    *reinterpret_cast<uint4*>(B + canon(n, k0, S::KP)) =
-        __ldg(reinterpret_cast<const uint4*>(bop + size_t(n) * S::KP + k0));
-  }
-  // columns KF..KP of both tiles are never written by a job
-  for (int b = threadIdx.x * 16; b < 2 * S::A96_BYTES; b += kFwdThreads * 16)
-    *reinterpret_cast<uint4*>(smem + b) = make_uint4(0, 0, 0, 0);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem0 = tslot;
-  const uint32_t idesc = idesc_bf16(S::NP);
-  uint32_t ph = 0u;  // bit b: the mbarrier phase to wait for on buffer b
-  int prev = -1;     // the tile whose MMAs are in flight
-  for (int tile = blockIdx.x, it = 0;; tile += gridDim.x, ++it) {
-    const bool have = tile < ntiles;
-    const int sb = it & 1;
-    if (have) a_tile_job<CIN, S::KP>(G, in, fwd_tile_site0(G, tile) + lane, lane, warp, abuf(sb));
-    fence_async_smem();
-    __syncthreads();
-    tc_fence_after();
-    if (prev >= 0) {
-      // the previous tile: wait for its MMAs (bounded), read its accumulator back
-      const int pb = sb ^ 1;
-      if (warp == 0) {
-        const bool ok = mbar_wait_bounded(&bar[pb], (ph >> pb) & 1u);
-        if (lane == 0) {
-          mma_ok = ok ? 1 : 0;
-          if (!ok) atomicExch(G.err, 1);
-        }
-      }
-      tc_fence_before();
-      __syncthreads();
-      tc_fence_after();
-      ph ^= 1u << pb;
-      if (!mma_ok) break;  // the same flag in every thread: the CTA leaves together
-    }
-    // This tile's MMAs go out before the previous tile is read back, so that
-    // the read-back overlaps them (the two use different accumulators; A of
-    // this tile and its accumulator were last used two tiles ago, which the
-    // barriers above have ordered).
-    if (have && threadIdx.x == 0) {
-      const uint32_t a0 = smem_u32(abuf(sb)), b0 = smem_u32(B);
-      constexpr uint32_t sbo = (S::KP / 8) * 128;
-#pragma unroll 1
-      for (int kb = 0; kb < S::KP / 16; ++kb)
-        umma_bf16(tmem0 + uint32_t(sb * S::TCOLS), smem_desc(a0 + kb * 256, 128, sbo),
-                  smem_desc(b0 + kb * 256, 128, sbo), idesc, kb > 0 ? 1u : 0u);
-      umma_commit(&bar[sb]);
-    }
-    if (prev >= 0 && warp < 3) {
-      const int pb = sb ^ 1;
-      const int r = warp * 32 + lane;
-      float v[S::NP];
-#pragma unroll
-      for (int c = 0; c < S::NP; c += 16)
-        tmem_ld16(tmem0 + uint32_t(pb * S::TCOLS) + (uint32_t(warp * 32) << 16) + c, v + c);
-      const int sl = r / 3, a = r - sl * 3;
-      const int s = fwd_tile_site0(G, prev) + sl;
-      if (s < G.V) {
-        float4* o4 = reinterpret_cast<float4*>(out) + size_t(a) * G.V + s;
-#pragma unroll
-        for (int q = 0; q < COUT / 2; ++q)
-          o4[size_t(3 * q) * G.V] = make_float4(v[4 * q], v[4 * q + 2], v[4 * q + 1], v[4 * q + 3]);
-      }
-    }
-    // the read-back's tensor-memory loads are ordered before the next
-    // iteration's barrier, after which that accumulator is written again
-    tc_fence_before();
-    if (!have) break;
-    prev = tile;
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem0, 2 * S::TCOLS);
-}
+constexpr int kDbThreads = 288;
 
 // ---- backward: dB[n][k] = sum over rows (site, colour) of dY[row][n] A[row][k] ------
 // ldmatrix, four 8x8 BF16 matrices transposed: lane l gives the address of row
@@ -582,7 +252,7 @@ struct PtcDb {
 };
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kFwdThreads, 2) ptc_db_kernel(PtcGeo G, const float2* __restrict__ in,
+__global__ void __launch_bounds__(kDbThreads, 2) ptc_db_kernel(PtcGeo G, const float2* __restrict__ in,
                                                              const float2* __restrict__ dy,
                                                              float* __restrict__ partial, int ntiles) {
   using S = PtcDb<CIN, COUT>;
@@ -591,7 +261,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ptc_db_kernel(PtcGeo G, const 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   unsigned char* As = smem + 6 * S::Y_BYTES + warp * S::A_BYTES;
   // the padding columns of dY (COUT = 4: 8 of 16) stay zero
-  for (int b = threadIdx.x * 16; b < 6 * S::Y_BYTES; b += kFwdThreads * 16)
+  for (int b = threadIdx.x * 16; b < 6 * S::Y_BYTES; b += kDbThreads * 16)
     *reinterpret_cast<uint4*>(smem + b) = make_uint4(0, 0, 0, 0);
   __syncthreads();
   float acc[S::MT][S::NH * S::NT][4];
@@ -611,7 +281,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ptc_db_kernel(PtcGeo G, const 
     unsigned char* Y = smem + (it & 1) * 3 * S::Y_BYTES;
     // dY of the tile: float4 row (3q + colour) of 32 sites -> columns 4q .. 4q+3
     // (re 2q, re 2q+1, im 2q, im 2q+1) of rows 32 colour + site
-    for (int j = threadIdx.x; j < 32 * 3 * (COUT / 2); j += kFwdThreads) {
+    for (int j = threadIdx.x; j < 32 * 3 * (COUT / 2); j += kDbThreads) {
       const int sl = j & 31, qa = j >> 5;
       const int q = qa / 3, a = qa - 3 * q;
       const float4 v = __ldg(reinterpret_cast<const float4*>(dy) + size_t(qa) * G.V + site0 + sl);
@@ -740,6 +410,284 @@ __global__ void feat_to_spinor_kernel(int Vh, const float2* feat, SpinorPtr e, S
   }
 }
 
+// ---- warp-level layer ----------------------------------------------------------------------
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t r[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+// c (16x8, FP32) += a (16x8) b (8x8), BF16
+__device__ __forceinline__ void mma_1688(float c[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(b0));
+}
+
+template <int CIN, int COUT>
+struct PtcLayer {
+  static constexpr int CH = CIN < 8 ? CIN : 8;    // channels transported at a time
+  static constexpr int NH = CIN / CH;
+  static constexpr int NB = CH == 8 ? 2 : 1;      // weight words per MMA (K = 16 or 8)
+  static constexpr int NT = 2 * COUT / 8;         // 8-column output tiles
+  static constexpr int AS = CH == 8 ? 48 : 16;    // bytes of a staged row (padded: conflict-free)
+  static constexpr int A_BYTES = 96 * AS;         // the three colours of a warp's 32 sites
+  static constexpr int WORDS = 9 * NH * NT * NB * 32;
+  // the next direction's loads: in registers (few channels), or requested into
+  // L1 (more); with 4 -> 16 channels the accumulators leave no registers for it
+  static constexpr bool RAW = CIN == 4 && NT <= 2;
+  static constexpr bool AHEAD = CIN >= 8;
+  static constexpr int THREADS = NT == 1 && CIN < 16 ? 512 : NT == 4 && CIN >= 8 ? 256 : 384;
+  static constexpr int SMEM = WORDS * 4 + (THREADS / 32) * A_BYTES;
+};
+
+// The channels of displacement D at one site, transported, as BF16 rows of the
+// warp's staging tile: row 32 colour + lane holds the real parts of the
+// channels, then the imaginary parts.  Then their product with the weights.
+// The feature rows and links of the next direction, requested into L1 while the
+// present one is multiplied: the loads of a direction wait ~7 issue slots per
+// instruction on L2 otherwise (long scoreboard; 20 warps an SM).
+template <int CIN, int KIND>
+__device__ __forceinline__ void prefetch_dir(const PtcGeo& G, const float2* __restrict__ in, int p, int hs, int mu,
+                                             int nb) {
+  const float4* f4 = reinterpret_cast<const float4*>(in) + ((1 - p) * G.g.Vh + nb);
+#pragma unroll
+  for (int q = 0; q < 3 * CIN / 2; ++q) asm volatile("prefetch.global.L1 [%0];" ::"l"(f4 + size_t(q) * G.V));
+  const float4* u = link_chunk0<3>(static_cast<const float4*>(G.gauge.a), G.g.Vh, KIND == 1 ? p : 1 - p, mu,
+                                   KIND == 1 ? hs : nb);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) asm volatile("prefetch.global.L1 [%0];" ::"l"(u + 32 * k));
+}
+
+// The loads of one direction (4 input channels), kept in registers while the
+// direction before is multiplied
+struct RawDir {
+  float4 f[6], u[3];
+};
+template <int KIND>
+__device__ __forceinline__ void load_dir4(const PtcGeo& G, const float2* __restrict__ in, int p, int hs, int mu, int nb,
+                                          RawDir& r) {
+  const float4* f4 = reinterpret_cast<const float4*>(in) + (KIND == 0 ? p * G.g.Vh + hs : (1 - p) * G.g.Vh + nb);
+#pragma unroll
+  for (int k = 0; k < 6; ++k) r.f[k] = __ldg(f4 + size_t(k) * G.V);
+  if (KIND != 0) {
+    const float4* u = link_chunk0<3>(static_cast<const float4*>(G.gauge.a), G.g.Vh, KIND == 1 ? p : 1 - p, mu,
+                                     KIND == 1 ? hs : nb);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) r.u[k] = __ldg(u + 32 * k);
+  }
+}
+template <int COUT, int KIND>
+__device__ __forceinline__ void mul_dir4(const RawDir& r, int D, const uint32_t* W, unsigned char* As, uint32_t a_addr,
+                                         float acc[6][PtcLayer<4, COUT>::NT][4]) {
+  using S = PtcLayer<4, COUT>;
+  const int lane = threadIdx.x & 31;
+  Su3<float> U;
+  if (KIND != 0) {
+    U.e[0][0] = {r.u[0].x, r.u[0].y};
+    U.e[0][1] = {r.u[0].z, r.u[0].w};
+    U.e[0][2] = {r.u[1].x, r.u[1].y};
+    U.e[1][0] = {r.u[1].z, r.u[1].w};
+    U.e[1][1] = {r.u[2].x, r.u[2].y};
+    U.e[1][2] = {r.u[2].z, r.u[2].w};
+    reconstruct_row2(U);
+  }
+  uint32_t wre[3][2], wim[3][2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const float4 a = r.f[3 * q], b = r.f[3 * q + 1], e = r.f[3 * q + 2];
+    const Cp h0 = {make_float2(a.x, a.y), make_float2(a.z, a.w)};
+    const Cp h1 = {make_float2(b.x, b.y), make_float2(b.z, b.w)};
+    const Cp h2 = {make_float2(e.x, e.y), make_float2(e.z, e.w)};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      Cp w;
+      if (KIND == 0) w = c == 0 ? h0 : (c == 1 ? h1 : h2);
+      else w = su3_row<KIND == 2>(U, c, h0, h1, h2);
+      const __nv_bfloat162 br = __floats2bfloat162_rn(w.re.x, w.re.y);
+      const __nv_bfloat162 bi = __floats2bfloat162_rn(w.im.x, w.im.y);
+      wre[c][q] = *reinterpret_cast<const uint32_t*>(&br);
+      wim[c][q] = *reinterpret_cast<const uint32_t*>(&bi);
+    }
+  }
+  __syncwarp();  // the staged rows of the previous product are read
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    *reinterpret_cast<uint4*>(As + (32 * c + lane) * S::AS) = make_uint4(wre[c][0], wre[c][1], wim[c][0], wim[c][1]);
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    uint32_t a[4];
+    ldsm4(a_addr + 32 * c * S::AS, a);
+#pragma unroll
+    for (int n = 0; n < S::NT; ++n) {
+      const uint32_t b = W[(D * S::NT + n) * 32 + lane];
+      mma_1688(acc[2 * c][n], a[0], a[1], b);
+      mma_1688(acc[2 * c + 1][n], a[2], a[3], b);
+    }
+  }
+}
+
+// KIND 0: the site itself; 1: forward, 2: backward along mu (a run-time index:
+// one copy of the code per kind, and no direction's loads hoisted over
+// another's, which spilled)
+template <int CIN, int COUT, int KIND>
+__device__ __forceinline__ void layer_dir(const PtcGeo& G, const float2* __restrict__ in, int p, int hs, int mu, int nb,
+                                          const uint32_t* W, unsigned char* As, uint32_t a_addr,
+                                          float acc[6][PtcLayer<CIN, COUT>::NT][4]) {
+  using S = PtcLayer<CIN, COUT>;
+  const int lane = threadIdx.x & 31;
+  const int D = KIND == 0 ? 0 : 2 * mu + KIND;
+  const size_t V = size_t(G.V);
+  const float4* f4 = reinterpret_cast<const float4*>(in) + (KIND == 0 ? p * G.g.Vh + hs : (1 - p) * G.g.Vh + nb);
+  Su3<float> U;
+  if (KIND == 1) GaugeIO<PREC_SINGLE, 12>::load(G.gauge, p, mu, hs, U);
+  if (KIND == 2) GaugeIO<PREC_SINGLE, 12>::load(G.gauge, 1 - p, mu, nb, U);
+#pragma unroll
+  for (int h = 0; h < S::NH; ++h) {
+    uint32_t wre[3][S::CH / 2], wim[3][S::CH / 2];
+#pragma unroll
+    for (int q = 0; q < S::CH / 2; ++q) {
+      const float4* f = f4 + size_t(3 * (q + 4 * h)) * V;
+      const float4 a = __ldg(f), b = __ldg(f + V), e = __ldg(f + 2 * V);
+      const Cp h0 = {make_float2(a.x, a.y), make_float2(a.z, a.w)};
+      const Cp h1 = {make_float2(b.x, b.y), make_float2(b.z, b.w)};
+      const Cp h2 = {make_float2(e.x, e.y), make_float2(e.z, e.w)};
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        Cp w;
+        if (KIND == 0) w = r == 0 ? h0 : (r == 1 ? h1 : h2);
+        else w = su3_row<KIND == 2>(U, r, h0, h1, h2);
+        const __nv_bfloat162 br = __floats2bfloat162_rn(w.re.x, w.re.y);
+        const __nv_bfloat162 bi = __floats2bfloat162_rn(w.im.x, w.im.y);
+        wre[r][q] = *reinterpret_cast<const uint32_t*>(&br);
+        wim[r][q] = *reinterpret_cast<const uint32_t*>(&bi);
+      }
+    }
+    __syncwarp();  // the staged rows of the previous product are read
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      unsigned char* row = As + (32 * r + lane) * S::AS;
+      if constexpr (S::CH == 4) {
+        *reinterpret_cast<uint4*>(row) = make_uint4(wre[r][0], wre[r][1], wim[r][0], wim[r][1]);
+      } else {
+        *reinterpret_cast<uint4*>(row) = make_uint4(wre[r][0], wre[r][1], wre[r][2], wre[r][3]);
+        *reinterpret_cast<uint4*>(row + 16) = make_uint4(wim[r][0], wim[r][1], wim[r][2], wim[r][3]);
+      }
+    }
+    __syncwarp();
+    uint32_t b[S::NT][S::NB];
+#pragma unroll
+    for (int n = 0; n < S::NT; ++n)
+#pragma unroll
+      for (int k = 0; k < S::NB; ++k) b[n][k] = W[(((D * S::NH + h) * S::NT + n) * S::NB + k) * 32 + lane];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      if constexpr (S::CH == 4) {
+        uint32_t a[4];
+        ldsm4(a_addr + 32 * r * S::AS, a);
+#pragma unroll
+        for (int n = 0; n < S::NT; ++n) {
+          mma_1688(acc[2 * r][n], a[0], a[1], b[n][0]);
+          mma_1688(acc[2 * r + 1][n], a[2], a[3], b[n][0]);
+        }
+      } else {
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          uint32_t a[4];
+          ldsm4(a_addr + (32 * r + 16 * m) * S::AS, a);
+#pragma unroll
+          for (int n = 0; n < S::NT; ++n) mma_16816(acc[2 * r + m][n], a, b[n][0], b[n][S::NB - 1]);
+        }
+      }
+    }
+  }
+}
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(PtcLayer<CIN, COUT>::THREADS, 1)
+    ptc_layer_kernel(PtcGeo G, const float2* __restrict__ in, float2* __restrict__ out,
+                     const __nv_bfloat16* __restrict__ bop, int ntiles) {
+  if (G.skip && *G.skip) return;
+  using S = PtcLayer<CIN, COUT>;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  uint32_t* W = reinterpret_cast<uint32_t*>(smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned char* As = smem + S::WORDS * 4 + warp * S::A_BYTES;
+  // the weights in the order of the MMA's B fragments: lane l of word k of
+  // (displacement d, channel block h, tile n) holds two consecutive k of
+  // output row 8n + l/4
+  constexpr int KP = Ptc<CIN, COUT>::KP;
+  for (int i = threadIdx.x; i < S::WORDS; i += S::THREADS) {
+    const int l = i & 31, k = (i >> 5) % S::NB, n = (i >> 5) / S::NB % S::NT;
+    const int dh = (i >> 5) / (S::NB * S::NT), d = dh / S::NH, h = dh % S::NH;
+    const int part = S::CH == 8 ? k : (l & 3) >> 1;
+    const int ch = S::CH == 8 ? 8 * h + 2 * (l & 3) : 2 * (l & 1);
+    W[i] = __ldg(reinterpret_cast<const uint32_t*>(bop + size_t(8 * n + (l >> 2)) * KP + (2 * d + part) * CIN + ch));
+  }
+  __syncthreads();
+  const int lj = lane >> 3, lr = lane & 7;
+  const uint32_t a_addr = smem_u32(As) + (S::CH == 4 ? uint32_t((8 * lj + lr) * S::AS)
+                                                     : uint32_t((8 * (lj & 1) + lr) * S::AS + 16 * (lj >> 1)));
+  constexpr int NW = S::THREADS / 32;
+  for (int tile = blockIdx.x * NW + warp; tile < ntiles; tile += gridDim.x * NW) {
+    const int p = tile & 1, hs = (tile >> 1) * kFwdSites + lane;
+    const Coord c = coord_of(G.g, hs, p);
+    int nb[8];
+    neighbours(G.g, c, hs, nb);
+    float acc[6][S::NT][4];
+#pragma unroll
+    for (int m = 0; m < 6; ++m)
+#pragma unroll
+      for (int n = 0; n < S::NT; ++n)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[m][n][k] = 0.f;
+    if constexpr (S::RAW) {
+      RawDir ra, rb;
+      load_dir4<0>(G, in, p, hs, 0, 0, ra);
+      load_dir4<1>(G, in, p, hs, 0, nb[0], rb);
+      mul_dir4<COUT, 0>(ra, 0, W, As, a_addr, acc);
+#pragma unroll 1
+      for (int mu = 0; mu < 4; ++mu) {
+        load_dir4<2>(G, in, p, hs, mu, mu == 0 ? nb[1] : mu == 1 ? nb[3] : mu == 2 ? nb[5] : nb[7], ra);
+        mul_dir4<COUT, 1>(rb, 2 * mu + 1, W, As, a_addr, acc);
+        if (mu < 3) load_dir4<1>(G, in, p, hs, mu + 1, mu == 0 ? nb[2] : mu == 1 ? nb[4] : nb[6], rb);
+        mul_dir4<COUT, 2>(ra, 2 * mu + 2, W, As, a_addr, acc);
+      }
+    } else {
+      if constexpr (S::AHEAD) prefetch_dir<CIN, 1>(G, in, p, hs, 0, nb[0]);
+      layer_dir<CIN, COUT, 0>(G, in, p, hs, 0, 0, W, As, a_addr, acc);
+#pragma unroll 1
+      for (int mu = 0; mu < 4; ++mu) {
+        const int nf = mu == 0 ? nb[0] : mu == 1 ? nb[2] : mu == 2 ? nb[4] : nb[6];
+        const int nr = mu == 0 ? nb[1] : mu == 1 ? nb[3] : mu == 2 ? nb[5] : nb[7];
+        if constexpr (S::AHEAD) prefetch_dir<CIN, 2>(G, in, p, hs, mu, nr);
+        layer_dir<CIN, COUT, 1>(G, in, p, hs, mu, nf, W, As, a_addr, acc);
+        if (S::AHEAD && mu < 3) prefetch_dir<CIN, 1>(G, in, p, hs, mu + 1, mu == 0 ? nb[2] : mu == 1 ? nb[4] : nb[6]);
+        layer_dir<CIN, COUT, 2>(G, in, p, hs, mu, nr, W, As, a_addr, acc);
+      }
+    }
+    // Lane (g, t) = (lane / 4, lane % 4) holds channel 4n + t of rows g and
+    // g + 8; neighbouring lanes exchange one row each, so that every lane has
+    // both channels of a pair for one row and stores them as one float4.
+    const int t = lane & 3;
+    const bool odd = t & 1;
+    float4* o4 = reinterpret_cast<float4*>(out) + (p * G.g.Vh + (tile >> 1) * kFwdSites + (lane >> 2) + (odd ? 8 : 0));
+#pragma unroll
+    for (int m = 0; m < 6; ++m)
+#pragma unroll
+      for (int n = 0; n < S::NT; ++n) {
+        const float* v = acc[m][n];
+        const float r0 = __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[2], 1);
+        const float r1 = __shfl_xor_sync(0xffffffffu, odd ? v[1] : v[3], 1);
+        const int q = 2 * n + (t >> 1);
+        o4[size_t(3 * q + m / 2) * G.V + 16 * (m & 1)] =
+            odd ? make_float4(r0, v[2], r1, v[3]) : make_float4(v[0], r0, v[1], r1);
+      }
+  }
+}
+
 // ---- host launchers ------------------------------------------------------------------
 static int sm_count() {
   static int n = 0;
@@ -752,63 +700,21 @@ static int sm_count() {
   return n;
 }
 
-// CTAs of `threads` threads of kernel f that fit on one SM by registers (65536
-// per SM, allocated per warp in units of 256): the persistent forward kernels
-// launch no more than this many per SM, so that no CTA waits for another to
-// finish before it starts its share of the tiles
-static int fit_by_registers(const void* f, int threads) {
-  cudaFuncAttributes a;
-  if (cudaFuncGetAttributes(&a, f) != cudaSuccess || a.numRegs <= 0) return 1 << 20;
-  const int per_warp = (a.numRegs * 32 + 255) / 256 * 256;
-  const int n = 65536 / (per_warp * ((threads + 31) / 32));
-  return n > 0 ? n : 1;
-}
-
 template <int CIN, int COUT>
 static cudaError_t fwd_t(const PtcGeo& G, const float2* in, float2* out, const __nv_bfloat16* bop,
                          cudaStream_t st) {
-  using S = Ptc<CIN, COUT>;
-  const int ntiles2 = (G.V + kFwdSites - 1) / kFwdSites;
-  // double-buffered where two A tiles leave room for at least two CTAs per SM
-  // in ~200 KB of shared memory (CIN <= 8); one tile otherwise
-  const int smem2 = 2 * S::A96_BYTES + S::BF_BYTES;
-  if ((200 * 1024) / (smem2 + 1024) >= 2) {
-    static bool attr2 = false;
-    if (!attr2) {
-      cudaError_t e = cudaFuncSetAttribute(ptc_fwd2_kernel<CIN, COUT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
-      if (e != cudaSuccess) return e;
-      attr2 = true;
-    }
-    int per_sm = (200 * 1024) / (smem2 + 1024);
-    if (per_sm > 2048 / kFwdThreads) per_sm = 2048 / kFwdThreads;
-    const int regs = fit_by_registers(reinterpret_cast<const void*>(ptc_fwd2_kernel<CIN, COUT>), kFwdThreads);
-    if (per_sm > regs) per_sm = regs;
-    int grid = sm_count() * per_sm;
-    if (grid > ntiles2) grid = ntiles2;
-    ptc_fwd2_kernel<CIN, COUT><<<grid, kFwdThreads, smem2, st>>>(G, in, out, bop, ntiles2);
-    return cudaGetLastError();
-  }
-  const int smem = S::A96_BYTES + S::BF_BYTES;
+  using S = PtcLayer<CIN, COUT>;
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(ptc_fwd_kernel<CIN, COUT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(ptc_layer_kernel<CIN, COUT>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
     if (e != cudaSuccess) return e;
     attr = true;
   }
+  // one CTA per SM (its register budget), each warp looping over tiles
   const int ntiles = (G.V + kFwdSites - 1) / kFwdSites;
-  // persistent: as many CTAs as fit on the device (threads, and shared memory
-  // up to ~150 KB per SM so that the rest of the SM's 256 KB stays L1 cache
-  // for the neighbour gathers), at most one per tile
-  int per_sm = (150 * 1024) / (smem + 1024);
-  if (per_sm > 2048 / kFwdThreads) per_sm = 2048 / kFwdThreads;
-  const int regs = fit_by_registers(reinterpret_cast<const void*>(ptc_fwd_kernel<CIN, COUT>), kFwdThreads);
-  if (per_sm > regs) per_sm = regs;
-  if (per_sm < 1) per_sm = 1;
-  int grid = sm_count() * per_sm;
-  if (grid > ntiles) grid = ntiles;
-  ptc_fwd_kernel<CIN, COUT><<<grid, kFwdThreads, smem, st>>>(G, in, out, bop, ntiles);
+  const int grid = std::min((ntiles + S::THREADS / 32 - 1) / (S::THREADS / 32), sm_count());
+  ptc_layer_kernel<CIN, COUT><<<grid, S::THREADS, S::SMEM, st>>>(G, in, out, bop, ntiles);
   return cudaGetLastError();
 }
 
@@ -830,7 +736,7 @@ static cudaError_t db_t(const PtcGeo& G, const float2* in, const float2* dy, flo
     attr = true;
   }
   const int grid = db_grid(G.V);
-  ptc_db_kernel<CIN, COUT><<<grid, kFwdThreads, S::SMEM, st>>>(G, in, dy, partial,
+  ptc_db_kernel<CIN, COUT><<<grid, kDbThreads, S::SMEM, st>>>(G, in, dy, partial,
                                                                (G.V + kFwdSites - 1) / kFwdSites);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -1332,7 +1238,6 @@ struct iro_ptc {
   float2* g1 = nullptr;
   float* partial = nullptr;           // weight-gradient partials, one per CTA
   float* db = nullptr;                // every layer's dL/dB, consecutive
-  int* err = nullptr;
   double* lpart = nullptr;
   size_t maxc = 0;
 };
@@ -1392,12 +1297,11 @@ void unpack_grad(int cin, int cout, const float* dB, float* g) {
       }
 }
 
-PtcGeo make_geo(iro_ctx* c, int* err) {
+PtcGeo make_geo(iro_ctx* c) {
   PtcGeo G;
   G.g = geom(c);
   G.gauge = gauge_single(c);
   G.V = int(volume(c));
-  G.err = err;
   G.skip = nullptr;
   return G;
 }
@@ -1430,18 +1334,15 @@ int feat_to_field(iro_ctx* c, const float2* feat, DevField& f, const int* skip =
   return convert(c, *t, f);
 }
 
-int check_err(iro_ctx* c, iro_ptc* n) {
-  int e = 0;
-  LCK(cudaMemcpyAsync(&e, n->err, sizeof(int), cudaMemcpyDeviceToHost, stream(c)));
+int wait_done(iro_ctx* c) {
   LCK(cudaStreamSynchronize(stream(c)));
-  if (e) return set_error(c, IRO_TIMEOUT, "tensor-core wait timed out in the network kernels");
   return IRO_OK;
 }
 
 // act[0] must hold the input features; runs every layer
 // the network's layers on n->act[0]; nothing when `skip` is set and nonzero
 int forward(iro_ctx* c, iro_ptc* n, const int* skip = nullptr) {
-  PtcGeo G = make_geo(c, n->err);
+  PtcGeo G = make_geo(c);
   G.skip = skip;
   for (int l = 0; l < n->nl; ++l)
     LCK(launch_ptc_fwd(n->w[l], n->w[l + 1], G, n->act[l], n->act[l + 1], n->bop[l], stream(c)));
@@ -1494,8 +1395,6 @@ int iro_ptc_create(iro_ctx* c, int nlayers, const int* widths, iro_ptc** out) {
   LCK(cudaMalloc(&n->g1, V * maxc * 3 * sizeof(float2)));
   LCK(cudaMalloc(&n->db, gradn * sizeof(float)));
   LCK(cudaMalloc(&n->partial, size_t(db_grid(int(V))) * maxnk * sizeof(float)));
-  LCK(cudaMalloc(&n->err, sizeof(int)));
-  LCK(cudaMemset(n->err, 0, sizeof(int)));
   LCK(cudaMalloc(&n->lpart, sizeof(double) * 2 * loss_blocks()));
   *out = n.release();
   return IRO_OK;
@@ -1508,7 +1407,7 @@ int iro_ptc_destroy(iro_ptc* n) {
   for (void* p : n->bop) cudaFree(p);
   for (void* p : n->badj) cudaFree(p);
   for (float2* p : n->act) cudaFree(p);
-  void* ps[] = {n->g0, n->g1, n->db, n->partial, n->err, n->lpart};
+  void* ps[] = {n->g0, n->g1, n->db, n->partial, n->lpart};
   for (void* p : ps)
     if (p) cudaFree(p);
   delete n;
@@ -1548,7 +1447,7 @@ int iro_ptc_apply_field(iro_ctx* c, iro_ptc* n, const iro_field* in, iro_field* 
   LRC(field_to_feat(c, *fi, n->act[0]));
   LRC(forward(c, n));
   LRC(feat_to_field(c, n->act[n->nl], *fo));
-  return check_err(c, n);
+  return wait_done(c);
 }
 
 int iro_ptc_apply(iro_ctx* c, iro_ptc* n, const double* in, double* out) {
@@ -1564,7 +1463,7 @@ int iro_ptc_apply(iro_ctx* c, iro_ptc* n, const double* in, double* out) {
   LRC(import_field(c, in, true, *a));
   LRC(field_to_feat(c, *a, n->act[0]));
   LRC(forward(c, n));
-  LRC(check_err(c, n));
+  LRC(wait_done(c));
   LRC(feat_to_field(c, n->act[n->nl], *b));
   return export_field(c, *b, true, out);
 }
@@ -1596,9 +1495,9 @@ int iro_ptc_loss_grad(iro_ctx* c, iro_ptc* n, const iro_field* in, const iro_fie
     tt += part[2 * b + 1];
   }
   *loss = dd / tt;
-  if (!grad) return check_err(c, n);
+  if (!grad) return wait_done(c);
   LCK(launch_loss_grad(nel, n->act[n->nl], n->g1, float(2.0 / tt), n->g0, st));
-  PtcGeo G = make_geo(c, n->err);
+  PtcGeo G = make_geo(c);
   float2* dy = n->g0;
   float2* dx = n->g1;
   std::vector<size_t> goff(n->nl + 1, 0), boff(n->nl + 1, 0);
@@ -1616,7 +1515,7 @@ int iro_ptc_loss_grad(iro_ctx* c, iro_ptc* n, const iro_field* in, const iro_fie
   LCK(cudaMemcpyAsync(dB.data(), n->db, dB.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
   LCK(cudaStreamSynchronize(st));
   for (int l = 0; l < n->nl; ++l) unpack_grad(n->w[l], n->w[l + 1], dB.data() + boff[l], grad + goff[l]);
-  return check_err(c, n);
+  return wait_done(c);
 }
 
 // ---- flexible GCR on A = D^dag D with the network as right preconditioner ---------------
@@ -1777,7 +1676,7 @@ int iro_gcr_solve_field(iro_ctx* c, int op, double mass, double csw, const iro_p
   out->fallback = fallback;
   out->precond_applies = pcapplies;
   if (net) {
-    int e = check_err(c, const_cast<iro_ptc*>(net));
+    int e = wait_done(c);
     if (e) return e;
   }
   if (!converged) return set_error(c, IRO_NOT_CONVERGED, "GCR not converged");
