@@ -75,6 +75,7 @@ struct iro_ctx {
   double* partials = nullptr;
   unsigned* counter = nullptr;
   double* redout = nullptr;
+  unsigned* sync_words = nullptr;  // the small-lattice CG's barrier counter and error flag
   void* state = nullptr;  // CGState[16] or MSState
   int* done = nullptr;    // [16]
   void* h_pinned = nullptr;  // host mirror of state + done
@@ -784,6 +785,8 @@ int iro_ctx_create(const int L[4], int device, iro_ctx** out) {
     CK(cudaMalloc(&c->counter, sizeof(unsigned) * (1 + groups)));
     CK(cudaMemset(c->counter, 0, sizeof(unsigned) * (1 + groups)));
     CK(cudaMalloc(&c->redout, sizeof(double) * kPartialsPerBlock));
+    CK(cudaMalloc(&c->sync_words, 2 * sizeof(unsigned)));
+    CK(cudaMemset(c->sync_words, 0, 2 * sizeof(unsigned)));
     CK(cudaMalloc(&c->state, sizeof(MSState) > sizeof(CGState) * kMaxRhs ? sizeof(MSState) : sizeof(CGState) * kMaxRhs));
     CK(cudaMalloc(&c->done, sizeof(int) * 64));
     CK(cudaMemset(c->done, 0, sizeof(int) * 64));
@@ -805,7 +808,7 @@ int iro_ctx_destroy(iro_ctx* c) {
   for (auto& kv : c->ws) free_field(kv.second);
   void* ptrs[] = {c->raw, c->ga.d12, c->ga.d18, c->ga.s12, c->ga.h12a, c->ga.h12b, c->ga.h18a,
                   c->ga.h18b, c->d_maxdev,
-                  c->d_singular, c->stage, c->partials, c->counter, c->redout, c->state, c->done};
+                  c->d_singular, c->stage, c->partials, c->counter, c->redout, c->sync_words, c->state, c->done};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (int pr = 0; pr < 3; ++pr)
@@ -1326,6 +1329,19 @@ int clover_ready(iro_ctx* c, double mass, double csw) { return ensure_clover(c, 
 GaugePtr gauge_double(iro_ctx* c) { return gauge_ptr(c, PREC_DOUBLE); }
 int gauge_recon(iro_ctx* c) { return c->recon; }
 const double2* gauge_d18(iro_ctx* c) { return c->ga.d18; }
+// the links the small-lattice CG reads: three stored rows in FP64 and FP16
+GaugePtr gauge_small(iro_ctx* c, int prec) {
+  GaugePtr g = gauge_ptr(c, prec);
+  if (prec == PREC_DOUBLE) g.a = c->ga.d18;
+  if (prec == PREC_HALF) {
+    g.a = c->ga.h18a;
+    g.b = c->ga.h18b;
+  }
+  return g;
+}
+unsigned* sync_words(iro_ctx* c) { return c->sync_words; }
+double* partials(iro_ctx* c) { return c->partials; }
+int sm_count(iro_ctx* c) { return c->sms; }
 bool gauge_loaded(iro_ctx* c) { return c->has_gauge; }
 CloverPtr clover(iro_ctx* c, int prec, int p, bool inverse) { return clover_ptr(c, prec, p, inverse); }
 }  // namespace host

@@ -96,6 +96,25 @@ cudaError_t launch_cg_init(int prec, int64_t Vh, int nrhs, SpinorPtr b, SpinorPt
 cudaError_t launch_cg_p(int prec, int64_t Vh, int nrhs, SpinorPtr p, SpinorPtr r, SpinorPtr x,
                         const CGState* state, const int* done, cudaStream_t st);
 
+// CG iterations of a small lattice in one cooperative launch (cg_small.cu):
+// up to `iters` iterations from the state, until every right-hand side has
+// left; bar and err: zeroed counter and error flag (set when a wait gave up)
+struct CgSmallLaunch {
+  Geom g;
+  GaugePtr gauge;  // FP64 and FP16: the links with three stored rows
+  int full, clover;
+  CloverPtr A[2], Ainv;
+  double kappa;
+  const DevField *p, *q, *r, *x, *t;  // t: an odd field (Schur operators)
+  CGState* state;
+  int* done;
+  int max_iter, iters, sms;
+  double* partials;  // 2 * max(4, nrhs) doubles per block
+  unsigned* bar;
+  int* err;
+};
+cudaError_t launch_cg_small(const CgSmallLaunch& L, cudaStream_t st);
+
 // Multishift, vectors in FP64 or FP32 (prec), FP64 scalars:
 // x0 -= beta p0; r += beta (s + sigma0 p0); reduce |r|^2
 cudaError_t launch_ms_xr(int prec, int64_t Vh, SpinorPtr x0, SpinorPtr r, SpinorPtr p0, SpinorPtr s,

@@ -50,6 +50,10 @@ CloverPtr clover(iro_ctx* c, int prec, int p, bool inverse);
 GaugePtr gauge_double(iro_ctx* c);
 int gauge_recon(iro_ctx* c);
 const double2* gauge_d18(iro_ctx* c);
+GaugePtr gauge_small(iro_ctx* c, int prec);
+unsigned* sync_words(iro_ctx* c);
+double* partials(iro_ctx* c);
+int sm_count(iro_ctx* c);
 bool gauge_loaded(iro_ctx* c);
 const Geom& geom(iro_ctx* c);
 int64_t volume(iro_ctx* c);
@@ -127,6 +131,79 @@ int iterate(iro_ctx* c, int nrhs, int max_iter, bool use_graph, F body) {
   return rc;
 }
 
+// Whether a lattice's iterations run in one cooperative launch (cg_small.cu):
+// by its groups of 32 elements, 296 of which are resident at once (two blocks
+// per SM).  Solves to 1e-10, launched / in one launch, ms:
+//   FP64 Wilson:  8^3x16 full 512 groups 6.67 / 3.14, 12^3x16 full 864 8.24 / 7.11,
+//                 16^4 e/o 1024 4.46 / 4.72, 8^4 e/o 12 rhs 1024 3.91 / 4.27
+//   FP64 clover:  8^3x16 e/o 128 4.11 / 2.34, 12^3x16 432 4.28 / 4.03, 16^4 1024 6.4 / 10.6
+//   FP32 Wilson:  16^4 e/o 1024 5.37 / 4.55, 12^3x16 e/o 3 rhs 1383 5.55 / 5.42,
+//                 16^4 full 2048 10.68 / 10.65, 8^3x16 e/o 12 rhs 2048 5.95 / 6.68
+//   FP32 clover:  16^4 e/o 1024 6.17 / 5.53, 16^3x32 2048 8.86 / 10.32
+//   FP16 Wilson:  16^4 e/o 1024 4.96 / 4.69, 12^3x16 e/o 3 rhs 1383 5.44 / 5.83
+//   FP16 clover:  12^3x16 e/o 432 5.26 / 3.86, 16^4 1024 5.61 / 5.87
+bool cg_is_small(int op, int prec, int nrhs, int64_t half_volume) {
+  static const int limit[3][2] = {{888, 448}, {1480, 1184}, {1036, 740}};
+  const bool cl = op == IRO_OP_CLOVER_FULL || op == IRO_OP_CLOVER_SCHUR_EE;
+  const int S = 32 / nrhs;  // sites of a group
+  const int64_t groups = (op_is_full(op) ? 2 : 1) * ((half_volume + S - 1) / S);
+  return groups <= limit[prec][cl ? 1 : 0];
+}
+
+// Iterations from the device state until every right-hand side has left (or
+// paused): the inner loop of cg_double and cg_mixed on a small lattice.  A
+// launch is bounded to kSmallIters iterations (a few ms).
+constexpr int kSmallIters = 256;
+int iterate_small(iro_ctx* c, int op, double mass, const DevField* P, const DevField* Q, const DevField* R,
+                  const DevField* X, int max_iter) {
+  const bool cl = op == IRO_OP_CLOVER_FULL || op == IRO_OP_CLOVER_SCHUR_EE;
+  const int prec = P->prec, nrhs = P->nrhs;
+  cudaStream_t st = stream(c);
+  int rc = IRO_OK;
+  CgSmallLaunch L{};
+  L.g = geom(c);
+  L.gauge = gauge_small(c, prec);
+  L.full = op_is_full(op);
+  L.clover = cl;
+  if (cl) {
+    L.A[0] = clover(c, prec, 0, false);
+    if (L.full) L.A[1] = clover(c, prec, 1, false);
+    else L.Ainv = clover(c, prec, 1, true);
+  }
+  L.kappa = 0.5 / (4.0 + mass);
+  L.p = P;
+  L.q = Q;
+  L.r = R;
+  L.x = X;
+  if (!L.full) {
+    L.t = workspace(c, 1, prec, nrhs, 0, &rc);
+    if (!L.t) return rc;
+  }
+  L.state = static_cast<CGState*>(state(c));
+  L.done = done(c);
+  L.max_iter = max_iter;
+  L.iters = kSmallIters;
+  L.sms = sm_count(c);
+  L.partials = partials(c);
+  L.bar = sync_words(c);
+  L.err = reinterpret_cast<int*>(sync_words(c) + 1);
+  int* hpin = static_cast<int*>(pinned(c));
+  for (int64_t launched = 0;;) {
+    CK(launch_cg_small(L, st));
+    launched += kSmallIters;
+    CK(cudaMemcpyAsync(hpin, done(c), sizeof(int) * nrhs, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hpin + 16, L.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (hpin[16]) {
+      CK(cudaMemsetAsync(L.err, 0, sizeof(int), st));
+      return set_error(c, IRO_TIMEOUT, "a grid barrier of the small-lattice CG timed out");
+    }
+    bool left = true;
+    for (int r = 0; r < nrhs; ++r) left = left && hpin[r] != RUNNING;
+    if (left || launched >= max_iter) return IRO_OK;
+  }
+}
+
 // FP64 CG on D^dag D, Solver_CG::solve (lib/Solver/solver_CG.cpp:29-80).
 int cg_double(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* prm,
               const DevField* B, DevField* X, int nrhs, iro_solver_out* out) {
@@ -168,7 +245,10 @@ int cg_double(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* 
     }
     return IRO_OK;
   };
-  RC(iterate(c, nrhs, prm->max_iter, prm->use_graph != 0, body));
+  if (cg_is_small(op, PREC_DOUBLE, nrhs, vh(c)))
+    RC(iterate_small(c, op, mass, P, Q, R, X, prm->max_iter));
+  else
+    RC(iterate(c, nrhs, prm->max_iter, prm->use_graph != 0, body));
   // true residual |A x - b| / |b| (solver_CG.cpp:69-71)
   RC(apply(c, op, mass, csw, false, *X, *Q, nullptr, 0, nullptr));
   RC(apply(c, op, mass, csw, true, *Q, *S, nullptr, 0, nullptr));
@@ -905,8 +985,9 @@ int cg_mixed(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* p
     }
     return IRO_OK;
   };
+  const bool small = !shifted && cg_is_small(op, pl, nrhs, vh(c));
   cudaGraphExec_t exec = nullptr;
-  if (prm->use_graph && st != nullptr) {
+  if (!small && prm->use_graph && st != nullptr) {
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int brc = body(kChunk);
@@ -926,9 +1007,12 @@ int cg_mixed(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* p
   std::vector<int> hdone(nrhs), mask(nrhs);
   for (;;) {
     // inner iterations until some right-hand side pauses or all have left
+    if (small) RC(iterate_small(c, op, mass, Pl, Ql, Rl, Xl, prm->max_iter));
     for (;;) {
-      if (exec) CK(cudaGraphLaunch(exec, st));
-      else RC(body(kChunk));
+      if (!small) {
+        if (exec) CK(cudaGraphLaunch(exec, st));
+        else RC(body(kChunk));
+      }
       CK(cudaMemcpyAsync(hpin, done(c), sizeof(int) * nrhs, cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
       bool any_pause = false, all_left = true;

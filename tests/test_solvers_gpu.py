@@ -218,3 +218,53 @@ def test_multishift_stopped_mid_window_vs_oracle(port):
     x = x.reshape(shifts.size, -1)
     for k in range(shifts.size):
         assert rel(x[k], xo[k]) < 1e-10, k
+
+
+# Lattices whose iterations run in one cooperative launch: fewer groups of 32
+# elements than SMs, one and several groups per block, a last group that is not
+# full (nrhs 3, 5: 10 and 6 sites a group), and the launched iteration just
+# above the rule's limit.
+@pytest.mark.parametrize("inner", ["double", "single", "half"])
+@pytest.mark.parametrize("op,L,nrhs", [
+    ("wilson", [4, 4, 4, 8], 1), ("wilson", [8, 8, 8, 12], 1), ("wilson", [4, 6, 4, 4], 5),
+    ("wilson_eo", [4, 4, 4, 8], 16), ("wilson_eo", [12, 12, 12, 16], 1), ("wilson_eo", [6, 4, 4, 6], 3),
+    ("clover", [4, 4, 6, 4], 3), ("clover_eo", [2, 4, 4, 4], 12), ("clover_eo", [8, 8, 8, 16], 1),
+    ("clover_eo", [12, 12, 16, 16], 1)])
+def test_cg_small_lattices(op, L, nrhs, inner):
+    """The FP64 true residual of every solution, formed with the operators of
+    the launched path (a different kernel), reaches the goal and is the one
+    reported."""
+    V = int(np.prod(L))
+    u = ib.synth_gauge(L, 0.2, 311, gauge_transform=True)
+    c = ib.Context(L, 0)
+    m, csw = 0.5 / 0.12 - 4, 1.0
+    D = {"wilson": lambda: ib.Dirac_Wilson(m, u, ctx=c),
+         "wilson_eo": lambda: ib.Dirac_Wilson_EvenOdd(m, u, ctx=c),
+         "clover": lambda: ib.Dirac_Clover(ib.Dirac_Wilson(m, u, ctx=c), csw, u, ctx=c),
+         "clover_eo": lambda: ib.Dirac_Clover_EvenOdd(m, csw, u, ctx=c)}[op]()
+    n = D.fsize()
+    b = np.concatenate([ib.synth_gaussian(n // 24, 320 + r) for r in range(nrhs)])
+    x, outs, rc = ib.Solver_CG(1e-20, 3000, ib.Fopr_DdagD(D), inner=inner).solve_many(b, nrhs)
+    assert rc == ib.OK
+    for r in range(nrhs):
+        br, xr = b[r * n:(r + 1) * n], x[r * n:(r + 1) * n]
+        res = np.linalg.norm(br - D.mult_dag(D.mult(xr))) / np.linalg.norm(br)
+        assert res < 1.05 * TOL_RES and outs[r].diff < TOL_RES
+        assert abs(res - outs[r].diff) < 1e-12 + 1e-2 * outs[r].diff
+
+
+def test_cg_small_lattice_without_su3():
+    """Links that are not in SU(3) (FP64, full 3x3 storage) on a small lattice,
+    against the oracle's CG."""
+    import oracle
+    L = [4, 4, 4, 8]
+    V = int(np.prod(L))
+    u = 1.02 * ib.synth_gauge(L, 0.2, 331, gauge_transform=True)
+    c = ib.Context(L, 0)
+    m = 0.5 / 0.115 - 4
+    D = ib.Dirac_Wilson_EvenOdd(m, u, ctx=c)
+    b = ib.synth_gaussian(V // 2, 332)
+    x = np.empty_like(b)
+    out = ib.Solver_CG(1e-20, 3000, ib.Fopr_DdagD(D)).solve(x, b)
+    xo, it, _ = oracle.port().cg(L, u, oracle.WILSON_EO, m, 0.0, b, 1e-20, 3000)
+    assert abs(out.Iterations - it) <= 2 and rel(x, xo) < TOL_SOL
