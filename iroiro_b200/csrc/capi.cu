@@ -435,15 +435,36 @@ HopLaunch base_launch(iro_ctx* c, int prec, bool dag, int nrhs) {
 // even nrhs 4..9 (two right-hand sides per thread); FP16 10..12 (the
 // mixed-precision kernel on the FP16 links with three stored rows at 3, 4 or
 // 2 blocks per SM, any nrhs) and 13..14 (the same kernel on the 12-real FP16
-// links, row 2 rebuilt per link, at 3 or 4 blocks per SM).
-constexpr int kHopVariants = 15;
+// links, row 2 rebuilt per link, at 3 or 4 blocks per SM); FP32 15 (24 warps
+// per SM, any nrhs).  IRO_HOP_VARIANT counts modulo the first 15.
+constexpr int kHopForced = 15;
+constexpr int kHopVariants = 16;
 
 static bool variant_ok(const HopLaunch& L, int v) {
   if (v < 0 || v >= kHopVariants) return false;
+  if (v == 15) return L.prec == PREC_SINGLE;
   if (v < 4) return true;
   if (L.prec == PREC_DOUBLE) return v < 12 && (v < 6 || L.recon == 12);
   if (v < 10) return L.recon == 12 && L.nrhs % 2 == 0;
   return L.prec == PREC_HALF && L.recon == 12;
+}
+
+// Candidates that are not timed: the FP64 variants of 128-thread blocks a second
+// time; the two-row links for full-lattice FP64 launches without clover blocks of
+// 8 right-hand sides and more; the staged kernels 8 and 9, which never won a shape.
+// Rebuilding the third row per right-hand side won the tuner's few repeated
+// launches (two-row links of 12x20x28x44 about fit L2) and lost in a program's:
+// that lattice, variants 4 / 10, one field repeated and three in turn, 8
+// right-hand sides 370, 416 / 365, 361 us, 12 581, 658 / 556, 570 us.  At 6 they
+// tie (283 / 278 us in turn), below that the bytes decide (1: 56 / 63 us); e/o
+// launches tie at 8 and 12 and keep both.
+static bool worth_timing(const HopLaunch& L, int v, int block) {
+  if (L.prec == PREC_DOUBLE) {
+    if (block > 128 && (v % 6 == 4 || v % 6 == 5)) return false;
+    const bool clov = L.epi == EPI_SCALE_CLOV || L.epi == EPI_XPAY_CLOV;
+    return !(L.recon == 12 && v < 6 && L.nparity == 2 && L.nrhs >= 8 && !clov);
+  }
+  return v != 8 && v != 9;
 }
 
 static cudaError_t launch_variant(iro_ctx* c, HopLaunch L, cudaStream_t st) {
@@ -475,8 +496,8 @@ int launch_tuned(iro_ctx* c, HopLaunch L) {
     int v = 0, b = 256, g = 0;
     std::sscanf(forced, "%d,%d,%d", &v, &b, &g);
     if (L.prec == PREC_DOUBLE) v %= (L.recon == 12 ? 12 : 6);
-    else if (!variant_ok(L, v % kHopVariants)) v %= 4;
-    else v %= kHopVariants;
+    else if (!variant_ok(L, v % kHopForced)) v %= 4;
+    else v %= kHopForced;
     c->tuned[key] = Tune{v, b, g != 0};
     it = c->tuned.find(key);
   }
@@ -500,7 +521,7 @@ int launch_tuned(iro_ctx* c, HopLaunch L) {
     for (int v = 0; v < kHopVariants; ++v)
       for (int b : {256, 128})
         for (int g : {0, 1}) {
-          if (!variant_ok(L, v)) continue;
+          if (!variant_ok(L, v) || !worth_timing(L, v, b)) continue;
           T.variant = v;
           T.block_cap = b;
           T.grid_free = g;

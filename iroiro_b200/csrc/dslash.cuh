@@ -147,6 +147,7 @@ struct HopParams {
   Geom g;
   int p0;  // parity of the output sites handled by blockIdx.y == 0
   int nrhs;
+  FastDiv dn;  // division by nrhs
   SpinorPtr in[2], out[2], xin[2];  // indexed by blockIdx.y
   GaugePtr gauge;
   CloverPtr clov[2];
@@ -173,12 +174,15 @@ struct HopParams {
 // VAR bit 3 (FP16 only): the mixed-precision direction code of
 // dslash_mix.cuh on the links with three stored rows (RECON 18) or two
 // (RECON 12, row 2 rebuilt), at least three 256-thread blocks per SM (four
-// with bit 0, two with bit 1).
+// with bit 0, two with bit 1);
+// VAR bit 4 (FP32 only): at least three 256-thread blocks per SM (register
+// cap 80, 24 warps an SM: a 12-RHS hop at 24^3x48 0.272 ms, 0.364 ms at 128
+// registers).
 template <int VAR>
 struct HopBounds {
   static constexpr int threads = (VAR & 4) ? 128 : 256;
   static constexpr int blocks =
-      (VAR & 8) ? ((VAR & 1) ? 4 : ((VAR & 2) ? 2 : 3))
+      (VAR & 16) ? 3 : (VAR & 8) ? ((VAR & 1) ? 4 : ((VAR & 2) ? 2 : 3))
                 : ((VAR & 4) ? 3 : ((VAR & 1) ? 2 : 1));
 };
 
@@ -200,10 +204,11 @@ __global__ void __launch_bounds__(HopBounds<VAR>::threads, HopBounds<VAR>::block
   const int e0 = P.hs0 * nrhs;         // element index of the first output
   double red[3] = {0.0, 0.0, 0.0};
   // the grid stride is a multiple of nrhs, so each thread keeps one rhs
-  const int r = (nrhs == 1) ? 0 : int((blockIdx.x * blockDim.x + threadIdx.x) % unsigned(nrhs));
+  const unsigned t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = (nrhs == 1) ? 0 : int(t0 - fdiv(t0, P.dn) * unsigned(nrhs));
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nthreads; t += gridDim.x * blockDim.x) {
     const int tid = e0 + t;
-    const int hs = (nrhs == 1) ? tid : int(unsigned(tid) / unsigned(nrhs));
+    const int hs = (nrhs == 1) ? tid : int(fdiv(uint32_t(tid), P.dn));
     if (P.skip && P.skip[r]) continue;
     const Coord c = coord_of(P.g, hs, p);
     int nb[8];

@@ -2,6 +2,8 @@
 // storage precision so the instantiations compile in parallel.
 #pragma once
 
+#include <atomic>
+
 #include "dslash.cuh"
 #include "dslash_pair.cuh"
 #include "dslash_stage.cuh"
@@ -9,12 +11,38 @@
 
 namespace iro {
 
+// A capped grid is no larger than the blocks that are resident at once: a
+// thread loops over the sites anyway, and what is left over would run as a
+// further wave that fills the device only in part (the cap of 8 blocks per SM
+// was 1.3 to 4 times what the kernels' registers let in).  Operator
+// applications, cap / resident: full Wilson 12x20x28x44 FP64 0.0668 / 0.0508 ms,
+// 12 right-hand sides 0.586 / 0.486, FP16 0.199 / 0.167; e/o 32^3x64 FP16 with
+// 5 right-hand sides 0.641 / 0.576.
+template <auto Kernel>
+static int resident_grid(const LaunchCfg& c, const HopLaunch& L) {
+  if (L.grid_cap() != L.max_blocks) return c.grid;
+  static std::atomic<int> per_sm[9];  // of this kernel, by warps per block
+  const int w = (c.block + 31) / 32;
+  int n = per_sm[w].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, c.block, 0) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = 8;
+    }
+    per_sm[w].store(n, std::memory_order_relaxed);
+  }
+  // max_blocks is 8 per SM
+  const int fit = L.max_blocks / 8 * n / L.nparity;
+  return c.grid > fit ? (fit > 0 ? fit : 1) : c.grid;
+}
+
 template <int SP, int GP, int RECON, bool DAG, int EPI, int VAR>
 static cudaError_t hop_go(const HopLaunch& L, cudaStream_t st) {
   HopParams P;
   P.g = L.g;
   P.p0 = L.p0;
   P.nrhs = L.nrhs;
+  P.dn = make_fastdiv(uint32_t(L.nrhs));
   for (int i = 0; i < 2; ++i) {
     P.in[i] = L.in[i];
     P.out[i] = L.out[i];
@@ -36,6 +64,7 @@ static cudaError_t hop_go(const HopLaunch& L, cudaStream_t st) {
   LaunchCfg c = launch_cfg(P.nhs, L.nrhs, L.grid_cap(),
                            L.block_cap < HopBounds<VAR>::threads ? L.block_cap
                                                                  : HopBounds<VAR>::threads);
+  c.grid = resident_grid<hop_kernel<SP, GP, RECON, DAG, EPI, SP, VAR>>(c, L);
   // programmatic dependent launch: the blocks of this grid may be scheduled
   // while the previous kernel's last blocks retire (hop_kernel waits for
   // that kernel's completion before it reads anything), hiding the launch
@@ -81,6 +110,7 @@ static cudaError_t hop_go_pair(const HopLaunch& L, cudaStream_t st) {
       P.cr[i] = L.cr[i];
     }
     LaunchCfg c = launch_cfg(L.g.Vh, L.nrhs / 2, L.grid_cap(), L.block_cap);
+    c.grid = resident_grid<hop_pair_kernel<SP, DAG, EPI, VAR>>(c, L);
     dim3 grid(c.grid, L.nparity);
     hop_pair_kernel<SP, DAG, EPI, VAR><<<grid, c.block, 0, st>>>(P);
     return cudaGetLastError();
@@ -138,6 +168,7 @@ static cudaError_t hop_go_stage(const HopLaunch& L, cudaStream_t st) {
 // 4-7 two right-hand sides per thread with the register cap none / 128 /
 // 152 / 168, 8-9 the same with the neighbours staged through shared memory.
 // FP64: 4/5 the 168-register 128-thread hop_kernel (5 with the rolled loop).
+// FP32, any nrhs: 15 the 80-register hop_kernel.
 // FP16 on links with three stored rows (RECON 18): only 10/11/12, the
 // mixed-precision hop_kernel (VAR 8 / 9 / 10: 3 / 4 / 2 blocks per SM).
 // FP16 on the 12-real links: also 13/14, the mixed-precision hop_kernel with
@@ -184,6 +215,8 @@ static cudaError_t hop_var_more(const HopLaunch& L, cudaStream_t st) {
       case 9: return hop_go_stage<SP, RECON, DAG, EPI, 1>(L, st);
       default: break;
     }
+    if constexpr (SP == PREC_SINGLE)
+      if (L.variant == 15) return hop_go<SP, GP, RECON, DAG, EPI, 16>(L, st);
     if constexpr (SP == PREC_HALF && RECON == 12) {
       switch (L.variant) {
         case 13: return hop_go<SP, GP, RECON, DAG, EPI, 8>(L, st);

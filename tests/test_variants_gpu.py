@@ -90,3 +90,30 @@ def test_forced_variant(variant):
     for inner in ("single", "half"):
         cg = res[f"cg_{inner}"]
         assert cg["rc"] == 0 and cg["diff"] < TOL_RES and cg["sol"] < TOL_SOL, cg
+
+
+# The autotuned launches where a thread's loop over a capped grid ends in a
+# remainder (46080 sites a parity times the right-hand sides against the resident
+# blocks) and the division by nrhs is by a multiplier.  FP64 against one
+# right-hand side at a time: another variant may round differently, each output
+# a sum of 8 x 18 products of size <= 1, some 150 roundings of 1.1e-16.
+@pytest.mark.parametrize("nrhs", [1, 3, 7, 8, 12])
+@pytest.mark.parametrize("op", ["OP_WILSON_FULL", "OP_CLOVER_SCHUR_EE"])
+def test_capped_grids_and_divisions(op, nrhs):
+    import numpy as np
+
+    import iroiro_b200 as ib
+    L, code = [12, 16, 20, 24], getattr(ib, op)
+    n = int(np.prod(L)) // (1 if op.endswith("FULL") else 2)
+    c = ib.Context(L, 0)
+    c.upload_gauge(ib.synth_gauge(L, 0.2, 411, gauge_transform=True), force=True)
+    m, csw = 0.5 / 0.12 - 4, 1.0
+    f = np.stack([ib.synth_gaussian(n, 420 + r) for r in range(nrhs)])
+    ref = np.stack([c.apply(code, m, csw, 1, f[r], "double") for r in range(nrhs)])
+    for prec, tol in (("double", 150 * 1.1e-16), ("single", TOL_FP32), ("half", TOL_FP16)):
+        got = c.apply(code, m, csw, 1, f.ravel(), prec, nrhs=nrhs).reshape(nrhs, -1)
+        for r in range(nrhs):
+            assert np.linalg.norm(got[r] - ref[r]) < tol * np.linalg.norm(ref[r]), (prec, r)
+    if op == "OP_WILSON_FULL" and nrhs >= 8:
+        picked = [t["variant"] for t in c.autotune_report() if t["prec"] == 0 and t["nrhs"] == nrhs]
+        assert picked and min(picked) >= 6  # the three-row links
