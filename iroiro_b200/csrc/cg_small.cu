@@ -77,6 +77,10 @@ __device__ __forceinline__ SmallSite small_site(const CgSmallParams& P) {
   return s;
 }
 
+// One stencil of the operator over this block's groups, and the sum that its
+// reduction takes.  k 0: Schur's first stencil, into the odd t; k 1: its second,
+// or the full operator's both parities.  dag 0: D p into q; 1: D^dag q
+// subtracted, times alpha, from the residual.
 template <int SP>
 __device__ __forceinline__ double hop_phase(const CgSmallParams& P, SmallShared<typename SpinorIO<SP>::Real>& sm,
                                             const SmallSite& site, int k, int dag) {
