@@ -3,7 +3,6 @@
 // the Krylov solvers.  See include/iroiro_b200.h for the contract of each
 // entry point and the reference interface it replaces.
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -11,19 +10,15 @@
 #include <cstring>
 #include <map>
 #include <memory>
-#include <mutex>
 #include <string>
-#include <thread>
 #include <tuple>
 #include <vector>
 
+#include "host_copy.h"
 #include "internal.h"
 #include "iroiro_b200.h"
 
 using namespace iro;
-
-// host threads of a copy to or from pageable memory (ring_copy)
-constexpr int kCopyThreads = 8;
 
 struct iro_field {
   iro_ctx* ctx;
@@ -160,32 +155,7 @@ DevField* ws(iro_ctx* c, int subset, int prec, int nrhs, int slot, int* rc) {
   return &(c->ws[key] = f);
 }
 
-// ---- host copies -----------------------------------------------------------------
-// The driver copies pageable host memory through its own staging on one host
-// thread (H2D ~21 GB/s; D2H into memory that was never touched 4.7 GB/s,
-// page faults included: 15.9 ms for the 75 MB force of a 16^3x32 lattice).
-// Copies to or from pageable memory of kRingMin bytes and more are split into
-// kRingSlot pieces that kCopyThreads host threads take in turn, each through
-// two pinned slots of its own: its DMAs overlap its host copies and those of
-// the other threads, and the page faults of a fresh destination are taken in
-// parallel.  The slots (16 MB in all) are small so that the pipeline fills at
-// once: with two 128 MB chunks the first DMA started after 4 ms of host
-// copying.  Pinned memory, device-accessible memory and small copies take the
-// direct DMA.  Measured: the 75 MB force D2H 15.9 -> 2.1 ms, its 50 MB of
-// inputs 1.9 -> 2.2 ms of DMA time but no driver staging; a 382 MB gauge
-// upload 13.5 -> 9.6 ms.
-constexpr size_t kRingSlot = size_t(1) << 20;
-constexpr size_t kRingMin = size_t(4) << 20;
-
-bool host_pageable(const void* p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return true;
-  }
-  return a.type == cudaMemoryTypeUnregistered;
-}
-
+// ---- host copies (host_copy.h) -----------------------------------------------------
 bool host_pinned(const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -195,130 +165,16 @@ bool host_pinned(const void* p) {
   return a.type == cudaMemoryTypeHost;
 }
 
-// The slots of one device, shared by its contexts: allocated by the first copy
-// that needs them, given back when the device's last context is destroyed.  One
-// copy at a time uses them; another one that comes meanwhile (from another
-// thread) takes the direct path.
-struct CopyRing {
-  std::mutex use;
-  char* buf = nullptr;
-  cudaEvent_t ev[2 * kCopyThreads] = {};  // a slot's last DMA
-  int contexts = 0;                       // guarded by g_ring_mutex
-};
-constexpr int kRingDevices = 16;
-CopyRing g_ring[kRingDevices];
-std::mutex g_ring_mutex;
-
-void ring_attach(int device) {
-  if (device < 0 || device >= kRingDevices) return;
-  std::lock_guard<std::mutex> lk(g_ring_mutex);
-  ++g_ring[device].contexts;
-}
-void ring_detach(int device) {
-  if (device < 0 || device >= kRingDevices) return;
-  std::lock_guard<std::mutex> lk(g_ring_mutex);
-  CopyRing& r = g_ring[device];
-  if (--r.contexts > 0) return;
-  if (r.buf) cudaFreeHost(r.buf);
-  r.buf = nullptr;
-  for (cudaEvent_t& e : r.ev) {
-    if (e) cudaEventDestroy(e);
-    e = nullptr;
-  }
-}
-
-int ensure_ring(iro_ctx* c, CopyRing& r) {
-  if (!r.buf) CK(cudaHostAlloc(reinterpret_cast<void**>(&r.buf), 2 * kCopyThreads * kRingSlot, cudaHostAllocDefault));
-  for (cudaEvent_t& e : r.ev)
-    if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  return IRO_OK;
-}
-
-// One thread's share of a copy between `host` and `dev` through slots 2w and
-// 2w + 1: pieces are taken from `next` until none is left.  A slot's event
-// marks its last DMA.
-cudaError_t ring_worker(iro_ctx* c, CopyRing& ring, int w, bool to_host, char* host, char* dev, size_t bytes,
-                        std::atomic<size_t>& next) {
-  cudaError_t e = cudaSetDevice(c->device);
-  if (e != cudaSuccess) return e;
-  char* slot[2] = {ring.buf + 2 * w * kRingSlot, ring.buf + (2 * w + 1) * kRingSlot};
-  cudaEvent_t ev[2] = {ring.ev[2 * w], ring.ev[2 * w + 1]};
-  const size_t none = ~size_t(0);
-  size_t off[2] = {none, none};  // device to host: the piece in flight in each slot
-  auto land = [&](int k) -> cudaError_t {
-    if (off[k] == none) return cudaSuccess;
-    const cudaError_t r = cudaEventSynchronize(ev[k]);
-    if (r == cudaSuccess) std::memcpy(host + off[k], slot[k], std::min(kRingSlot, bytes - off[k]));
-    off[k] = none;
-    return r;
-  };
-  for (int k = 0;; k ^= 1) {
-    if (to_host && (e = land(k)) != cudaSuccess) return e;
-    const size_t o = next.fetch_add(1) * kRingSlot;
-    if (o >= bytes) return to_host ? land(k ^ 1) : cudaSuccess;
-    const size_t len = std::min(kRingSlot, bytes - o);
-    if (to_host) {
-      e = cudaMemcpyAsync(slot[k], dev + o, len, cudaMemcpyDeviceToHost, c->stream);
-      off[k] = o;
-    } else {
-      // the slot's previous DMA (of this copy or an earlier one) is done
-      if ((e = cudaEventSynchronize(ev[k])) != cudaSuccess) return e;
-      std::memcpy(slot[k], host + o, len);
-      e = cudaMemcpyAsync(dev + o, slot[k], len, cudaMemcpyHostToDevice, c->stream);
-    }
-    if (e == cudaSuccess) e = cudaEventRecord(ev[k], c->stream);
-    if (e != cudaSuccess) return e;
-  }
-}
-
-int ring_copy(iro_ctx* c, CopyRing& ring, bool to_host, char* host, char* dev, size_t bytes) {
-  RCK(ensure_ring(c, ring));
-  std::atomic<size_t> next{0};
-  const int nt = int(std::min<size_t>(std::min<unsigned>(kCopyThreads, std::max(1u, std::thread::hardware_concurrency())),
-                                      (bytes + kRingSlot - 1) / kRingSlot));
-  cudaError_t err[kCopyThreads] = {};
-  std::vector<std::thread> th;
-  // a thread that cannot be created leaves its share to the others
-  try {
-    th.reserve(nt);
-    for (int w = 1; w < nt; ++w)
-      th.emplace_back([&, w] { err[w] = ring_worker(c, ring, w, to_host, host, dev, bytes, next); });
-  } catch (...) {
-  }
-  err[0] = ring_worker(c, ring, 0, to_host, host, dev, bytes, next);
-  for (auto& t : th) t.join();
-  for (cudaError_t e : err)
-    if (e != cudaSuccess) {
-      cudaStreamSynchronize(c->stream);  // nothing of a failed copy stays in flight
-      return cuda_fail(c, e, "host copy");
-    }
-  return IRO_OK;
-}
-
-// the ring, locked, if this copy goes through it
-CopyRing* ring_for(iro_ctx* c, const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
-  if (bytes < kRingMin || c->device < 0 || c->device >= kRingDevices || !host_pageable(host)) return nullptr;
-  lk = std::unique_lock<std::mutex>(g_ring[c->device].use, std::try_to_lock);
-  return lk.owns_lock() ? &g_ring[c->device] : nullptr;
-}
-
 // device -> host, returns with the copy complete
 int copy_d2h(iro_ctx* c, void* host, const void* dev, size_t bytes) {
-  std::unique_lock<std::mutex> lk;
-  if (CopyRing* r = ring_for(c, host, bytes, lk))
-    return ring_copy(c, *r, true, static_cast<char*>(host), const_cast<char*>(static_cast<const char*>(dev)), bytes);
-  CK(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(copy_to_host(c->device, c->stream, host, dev, bytes));
   return IRO_OK;
 }
 
-// host -> device, enqueued on the context's stream (the host buffer may be
+// host -> device, in order with the context's stream (the host buffer may be
 // reused once this returns)
 int copy_h2d(iro_ctx* c, void* dev, const void* host, size_t bytes) {
-  std::unique_lock<std::mutex> lk;
-  if (CopyRing* r = ring_for(c, host, bytes, lk))
-    return ring_copy(c, *r, false, const_cast<char*>(static_cast<const char*>(host)), static_cast<char*>(dev), bytes);
-  CK(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, c->stream));
+  CK(copy_to_device(c->device, c->stream, dev, host, bytes));
   return IRO_OK;
 }
 

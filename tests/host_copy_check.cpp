@@ -1,0 +1,143 @@
+// csrc/host_copy.h against a CUDA runtime of this file's own: device memory is
+// host memory, and a stream runs its queued operations only when an event
+// recorded in it, or the stream, is waited for: the latest moment that the
+// CUDA ordering rules allow.  argv[1] names the check; exits 0 when it holds.
+#include "host_copy.h"
+
+#include <cstdio>
+#include <cstdlib>
+#include <deque>
+#include <map>
+#include <string>
+
+namespace {
+
+struct Op {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+struct Stream {
+  std::deque<Op> queue;
+  size_t done = 0, queued = 0;
+};
+struct Event {
+  Stream* st = nullptr;
+  size_t at = 0;
+};
+std::mutex g_mutex;
+std::map<cudaStream_t, Stream> g_streams;
+bool g_fail_pinned = false;
+int g_pinned_live = 0, g_copies = 0;
+
+void run_until(Stream& s, size_t at) {
+  while (s.done < at) {
+    std::memcpy(s.queue.front().dst, s.queue.front().src, s.queue.front().bytes);
+    s.queue.pop_front();
+    ++s.done;
+  }
+}
+
+}  // namespace
+
+extern "C" {
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
+  a->type = cudaMemoryTypeUnregistered;
+  return cudaSuccess;
+}
+cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned) {
+  if (g_fail_pinned) return cudaErrorMemoryAllocation;
+  *p = std::malloc(bytes);
+  ++g_pinned_live;
+  return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void* p) {
+  std::free(p);
+  --g_pinned_live;
+  return cudaSuccess;
+}
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+  *e = reinterpret_cast<cudaEvent_t>(new Event);
+  return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+  delete reinterpret_cast<Event*>(e);
+  return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_mutex);
+  Stream& s = g_streams[st];
+  *reinterpret_cast<Event*>(e) = Event{&s, s.queued};
+  return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+  std::lock_guard<std::mutex> lk(g_mutex);
+  const Event& v = *reinterpret_cast<Event*>(e);
+  if (v.st) run_until(*v.st, v.at);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t bytes, cudaMemcpyKind, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_mutex);
+  Stream& s = g_streams[st];
+  s.queue.push_back(Op{dst, src, bytes});
+  ++s.queued;
+  ++g_copies;
+  return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_mutex);
+  Stream& s = g_streams[st];
+  run_until(s, s.queued);
+  return cudaSuccess;
+}
+}
+
+using namespace iro;
+using Bytes = std::vector<unsigned char>;
+
+static cudaStream_t stream(long k) { return reinterpret_cast<cudaStream_t>(0x1000 * k); }
+static Bytes pattern(size_t n, unsigned seed) {
+  Bytes b(n);
+  for (size_t i = 0; i < n; ++i) b[i] = static_cast<unsigned char>((i >> 8) * 37 + i + seed);
+  return b;
+}
+static int verdict(bool ok, const char* what) {
+  if (!ok) std::printf("%s\n", what);
+  return ok ? 0 : 1;
+}
+
+// An upload on one context's stream, then a download on another's: the second
+// copy's DMAs must not touch a slot before the first's have read it.
+static int other_context(size_t up, size_t down) {
+  const Bytes a = pattern(up, 1), b = pattern(down, 2);
+  Bytes dev_a(up), dev_b = b, host_b(down);
+  ring_attach(0);
+  ring_attach(0);
+  copy_to_device(0, stream(1), dev_a.data(), a.data(), up);
+  copy_to_host(0, stream(2), host_b.data(), dev_b.data(), down);
+  cudaStreamSynchronize(stream(1));
+  int rc = verdict(dev_a == a, "the upload was overwritten") + verdict(host_b == b, "wrong download");
+  // as two contexts are destroyed: the slots go with the last one
+  copy_to_device(0, stream(2), dev_b.data(), b.data(), down);
+  copy_to_device(0, stream(1), dev_a.data(), a.data(), up);
+  cudaStreamSynchronize(stream(1));
+  ring_detach(0);
+  cudaStreamSynchronize(stream(2));
+  ring_detach(0);
+  return rc + verdict(g_pinned_live == 0, "pinned slots kept") + verdict(dev_a == a && dev_b == b, "wrong uploads");
+}
+
+int main(int argc, char** argv) {
+  const std::string what = argc > 1 ? argv[1] : "";
+  const size_t MB = size_t(1) << 20;
+  if (what == "other_context") {
+    int rc = 0;
+    for (size_t up : {8 * MB, 16 * MB, 40 * MB + 24})
+      for (size_t down : {8 * MB, 16 * MB + 8, 64 * MB}) rc += other_context(up, down);
+    return rc;
+  }
+  std::printf("unknown check\n");
+  return 2;
+}

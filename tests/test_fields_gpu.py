@@ -66,3 +66,24 @@ def test_pageable_round_trip_around_the_threaded_copy(nrhs):
     for t in ts:
         t.join()
     assert not bad
+
+
+def test_upload_with_work_queued_before_another_context_copies():
+    """An upload whose DMAs wait behind work queued on its context, then copies
+    of a second context of the device: the first context's field is what was
+    uploaded, bit for bit."""
+    L = [8, 8, 8, 16]
+    V = int(np.prod(L))
+    u = ib.synth_gauge(L, 0.2, 61, gauge_transform=True)
+    a, b = ib.Context(L, 0), ib.Context(L, 0)
+    a.upload_gauge(u)
+    op = ib.Dirac_Wilson(0.5 / 0.12 - 4.0, u, ctx=a)
+    f, g = ib.synth_gaussian(V * 6, 62), ib.synth_gaussian(V * 12, 63)
+    fa, fb = ib.DeviceField(a, 2, "double", 6), ib.DeviceField(b, 2, "double", 12).upload(g)
+    src, dst = (ib.DeviceField(a, 2, "double", 12).upload(g) for _ in range(2))
+    for _ in range(20):
+        for _ in range(100):  # a few ms
+            a.check(ib.lib().iro_dirac_apply_field(a.h, op.op, op.mass, 0.0, 0, src.h, dst.h), "apply")
+        fa.upload(f)
+        assert np.array_equal(fb.download(), g)
+        assert np.array_equal(fa.download(), f)
