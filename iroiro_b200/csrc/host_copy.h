@@ -1,17 +1,15 @@
 // Copies between pageable host memory and a device through pinned slots.
 //
 // The driver copies pageable host memory through its own staging on one host
-// thread (H2D ~21 GB/s; D2H into memory that was never touched 4.7 GB/s,
-// page faults included: 15.9 ms for the 75 MB force of a 16^3x32 lattice).
-// Copies to or from pageable memory of kRingMin bytes and more are split into
-// kRingSlot pieces that kCopyThreads host threads take in turn, each through
-// two pinned slots of its own: its DMAs overlap its host copies and those of
-// the other threads, and the page faults of a fresh destination are taken in
-// parallel.  The slots (16 MB in all) are small so that the pipeline fills at
-// once: with two 128 MB chunks the first DMA started after 4 ms of host
-// copying.  Pinned memory, device-accessible memory and small copies take the
-// direct DMA.  Measured: the 75 MB force D2H 15.9 -> 2.1 ms, its 50 MB of
-// inputs 1.9 -> 2.2 ms of DMA time but no driver staging; a 382 MB gauge
+// thread, which also takes the page faults of a destination that was never
+// touched (15.9 ms for the 75 MB force of a 16^3x32 lattice).  A larger copy is
+// split into kRingSlot pieces that kCopyThreads host threads take in turn, each
+// through two pinned slots of its own: its DMAs overlap its host copies and
+// those of the other threads, and page faults are taken in parallel.  The slots
+// (16 MB in all) are small so that the pipeline fills at once: with two 128 MB
+// chunks the first DMA started after 4 ms of host copying.  Pinned memory,
+// device-accessible memory and the copies that ring_pays() leaves out take the
+// direct DMA.  The 75 MB force to the host 15.9 -> 2.1 ms; a 382 MB gauge
 // upload 13.5 -> 9.6 ms.
 //
 // Only the CUDA runtime's C interface is used, so that a CPU test can link
@@ -19,10 +17,13 @@
 #pragma once
 
 #include <cuda_runtime_api.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
 #include <cstddef>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <thread>
@@ -32,7 +33,6 @@ namespace iro {
 
 constexpr int kCopyThreads = 8;
 constexpr size_t kRingSlot = size_t(1) << 20;
-constexpr size_t kRingMin = size_t(4) << 20;
 
 inline bool host_pageable(const void* p) {
   cudaPointerAttributes a;
@@ -41,6 +41,34 @@ inline bool host_pageable(const void* p) {
     return true;
   }
   return a.type == cudaMemoryTypeUnregistered;
+}
+
+// Whether most of a destination's pages were never touched (no page is there
+// yet): 16 of them are looked at.
+inline bool host_untouched(const void* p, size_t bytes) {
+  const uintptr_t page = uintptr_t(sysconf(_SC_PAGESIZE)), a = reinterpret_cast<uintptr_t>(p);
+  int absent = 0;
+  for (int k = 0; k < 16; ++k) {
+    unsigned char v = 1;
+    const uintptr_t q = (a + bytes / 16 * k + bytes / 32) / page * page;
+    if (mincore(reinterpret_cast<void*>(q), page, &v) == 0 && !(v & 1)) ++absent;
+  }
+  return absent > 8;
+}
+
+// The copies that the slots make faster.  Starting the threads takes a
+// hundred microseconds or two, which a copy has to win back.  Slots / direct,
+// us (boxes differ by 10 %, by 25 % for the touched downloads):
+//   upload, source in cache      4 MB 264 / 237, 8 MB 413 / 403, 10 MB 474 / 499, 16 MB 627 / 851
+//   upload, source not in cache  4 MB 303 / 436, 8 MB 456 / 804, 10 MB 528 / 1011, 16 MB 686 / 1582
+//   download, touched            8 MB 661 / 465, 16 MB 1073 / 870, 24 MB 1334 / 1391, 32 MB 1499 / 1678
+//   download, untouched          4 MB 1175 / 1770, 16 MB 2655 / 7906, 64 MB 9264 / 32936
+constexpr size_t kRingUp = size_t(10) << 20;
+constexpr size_t kRingDown = size_t(32) << 20;
+constexpr size_t kRingDownUntouched = size_t(4) << 20;
+inline bool ring_pays(bool to_host, const void* host, size_t bytes) {
+  if (!to_host) return bytes >= kRingUp;
+  return bytes >= kRingDown || (bytes >= kRingDownUntouched && host_untouched(host, bytes));
 }
 
 // The slots of one device, shared by its contexts: allocated by the first copy
@@ -166,9 +194,9 @@ inline cudaError_t ring_copy(int device, cudaStream_t st, CopyRing& ring, bool t
 }
 
 // the ring, locked, if this copy goes through it
-inline CopyRing* ring_for(int device, const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
+inline CopyRing* ring_for(int device, bool to_host, const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
   CopyRing* r = ring_of(device);
-  if (bytes < kRingMin || !r || !host_pageable(host)) return nullptr;
+  if (!r || !ring_pays(to_host, host, bytes) || !host_pageable(host)) return nullptr;
   lk = std::unique_lock<std::mutex>(r->use, std::try_to_lock);
   return lk.owns_lock() ? r : nullptr;
 }
@@ -176,7 +204,7 @@ inline CopyRing* ring_for(int device, const void* host, size_t bytes, std::uniqu
 // device -> host, returns with the copy complete
 inline cudaError_t copy_to_host(int device, cudaStream_t st, void* host, const void* dev, size_t bytes) {
   std::unique_lock<std::mutex> lk;
-  if (CopyRing* r = ring_for(device, host, bytes, lk))
+  if (CopyRing* r = ring_for(device, true, host, bytes, lk))
     return ring_copy(device, st, *r, true, static_cast<char*>(host), const_cast<char*>(static_cast<const char*>(dev)),
                      bytes);
   const cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
@@ -187,7 +215,7 @@ inline cudaError_t copy_to_host(int device, cudaStream_t st, void* host, const v
 // reused once this returns)
 inline cudaError_t copy_to_device(int device, cudaStream_t st, void* dev, const void* host, size_t bytes) {
   std::unique_lock<std::mutex> lk;
-  if (CopyRing* r = ring_for(device, host, bytes, lk))
+  if (CopyRing* r = ring_for(device, false, host, bytes, lk))
     return ring_copy(device, st, *r, false, const_cast<char*>(static_cast<const char*>(host)), static_cast<char*>(dev),
                      bytes);
   return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);

@@ -129,15 +129,54 @@ static int other_context(size_t up, size_t down) {
   return rc + verdict(g_pinned_live == 0, "pinned slots kept") + verdict(dev_a == a && dev_b == b, "wrong uploads");
 }
 
+// What a copy queues: one operation when it is direct, one per MiB through the slots
+static int copies(bool up, void* host, size_t n) {
+  static Bytes dev(size_t(80) << 20);
+  const int before = g_copies;
+  if (up) copy_to_device(0, stream(1), dev.data(), host, n);
+  else copy_to_host(0, stream(1), host, dev.data(), n);
+  cudaStreamSynchronize(stream(1));
+  return g_copies - before;
+}
+
+// Which copies go through the slots: by direction, size and whether the
+// destination was touched before
+static int route() {
+  const size_t MB = size_t(1) << 20;
+  Bytes touched(80 * MB, 1);
+  int rc = 0;
+  ring_attach(0);
+  auto expect = [&](bool up, void* host, size_t n, bool slots, const char* what) {
+    const int k = copies(up, host, n), want = slots ? int((n + MB - 1) / MB) : 1;
+    if (k != want) std::printf("%zu bytes: %d operations instead of %d, ", n, k, want);
+    rc += verdict(k == want, what);
+  };
+  for (size_t n : {MB, 4 * MB, 8 * MB, 10 * MB - 8}) expect(true, touched.data(), n, false, "upload");
+  for (size_t n : {10 * MB, 17 * MB + 8, 64 * MB}) expect(true, touched.data(), n, true, "upload");
+  for (size_t n : {MB, 4 * MB, 16 * MB, 32 * MB - 8}) expect(false, touched.data(), n, false, "touched download");
+  for (size_t n : {32 * MB, 40 * MB + 8, 80 * MB}) expect(false, touched.data(), n, true, "touched download");
+  for (size_t n : {4 * MB - 8, 4 * MB, 8 * MB + 8, 24 * MB}) {
+    // any alignment, and memory that ends with the destination
+    const size_t room = (n + 8191) / 4096 * 4096;
+    char* p = static_cast<char*>(mmap(nullptr, room, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
+    expect(false, p + (room - n), n, n >= 4 * MB, "untouched download");
+    expect(false, p + (room - n), n, n >= 32 * MB, "the same again, touched now");
+    munmap(p, room);
+  }
+  ring_detach(0);
+  return rc;
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   const size_t MB = size_t(1) << 20;
   if (what == "other_context") {
     int rc = 0;
-    for (size_t up : {8 * MB, 16 * MB, 40 * MB + 24})
-      for (size_t down : {8 * MB, 16 * MB + 8, 64 * MB}) rc += other_context(up, down);
+    for (size_t up : {10 * MB, 16 * MB, 40 * MB + 24})
+      for (size_t down : {32 * MB, 33 * MB + 8, 64 * MB}) rc += other_context(up, down);
     return rc;
   }
+  if (what == "route") return route();
   std::printf("unknown check\n");
   return 2;
 }

@@ -40,13 +40,13 @@ def test_norm_and_dot(ctx, prec, tol):
     assert np.all(np.abs(da.dot(db) - ref) <= tol * np.linalg.norm(A, axis=1) * np.linalg.norm(B, axis=1))
 
 
-@pytest.mark.parametrize("nrhs", [2, 3, 5, 12])
+@pytest.mark.parametrize("nrhs", [2, 3, 5, 12, 13])
 def test_pageable_round_trip_around_the_threaded_copy(nrhs):
-    """Uploads and downloads below and above the size from which pageable
-    memory is copied by several threads in 1 MiB pieces (1.5 MiB per
-    right-hand side here: a direct copy, then whole and odd numbers of pieces),
+    """Uploads and downloads below and above the sizes from which pageable
+    memory is copied by several threads in 1 MiB pieces (3 MiB per right-hand
+    side here: direct copies, then pieces in one direction or both),
     bit for bit; again with two contexts copying from two threads at once."""
-    L = [8, 8, 8, 16]
+    L = [8, 8, 8, 32]
     n = int(np.prod(L)) * nrhs
     f = ib.synth_gaussian(n, 50 + nrhs)
     ctxs = [ib.Context(L, 0) for _ in range(2)]
@@ -72,17 +72,17 @@ def test_upload_with_work_queued_before_another_context_copies():
     """An upload whose DMAs wait behind work queued on its context, then copies
     of a second context of the device: the first context's field is what was
     uploaded, bit for bit."""
-    L = [8, 8, 8, 16]
+    L = [8, 8, 8, 32]
     V = int(np.prod(L))
     u = ib.synth_gauge(L, 0.2, 61, gauge_transform=True)
     a, b = ib.Context(L, 0), ib.Context(L, 0)
     a.upload_gauge(u)
     op = ib.Dirac_Wilson(0.5 / 0.12 - 4.0, u, ctx=a)
-    f, g = ib.synth_gaussian(V * 6, 62), ib.synth_gaussian(V * 12, 63)
-    fa, fb = ib.DeviceField(a, 2, "double", 6), ib.DeviceField(b, 2, "double", 12).upload(g)
+    f, g = ib.synth_gaussian(V * 11, 62), ib.synth_gaussian(V * 12, 63)
+    fa, fb = ib.DeviceField(a, 2, "double", 11), ib.DeviceField(b, 2, "double", 12).upload(g)
     src, dst = (ib.DeviceField(a, 2, "double", 12).upload(g) for _ in range(2))
     for _ in range(20):
-        for _ in range(100):  # a few ms
+        for _ in range(50):  # a few ms
             a.check(ib.lib().iro_dirac_apply_field(a.h, op.op, op.mass, 0.0, 0, src.h, dst.h), "apply")
         fa.upload(f)
         assert np.array_equal(fb.download(), g)
