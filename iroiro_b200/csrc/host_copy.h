@@ -169,8 +169,6 @@ inline cudaError_t ring_worker(int device, cudaStream_t st, CopyRing& ring, int 
 
 inline cudaError_t ring_copy(int device, cudaStream_t st, CopyRing& ring, bool to_host, char* host, char* dev,
                              size_t bytes) {
-  cudaError_t e = ensure_ring(ring);
-  if (e != cudaSuccess) return e;
   std::atomic<size_t> next{0};
   const int nt = int(std::min<size_t>(std::min<unsigned>(kCopyThreads, std::max(1u, std::thread::hardware_concurrency())),
                                       (bytes + kRingSlot - 1) / kRingSlot));
@@ -193,12 +191,16 @@ inline cudaError_t ring_copy(int device, cudaStream_t st, CopyRing& ring, bool t
   return cudaSuccess;
 }
 
-// the ring, locked, if this copy goes through it
+// the ring, locked, if this copy goes through it (not when its slots cannot be
+// allocated: the direct copy needs no pinned memory)
 inline CopyRing* ring_for(int device, bool to_host, const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
   CopyRing* r = ring_of(device);
   if (!r || !ring_pays(to_host, host, bytes) || !host_pageable(host)) return nullptr;
   lk = std::unique_lock<std::mutex>(r->use, std::try_to_lock);
-  return lk.owns_lock() ? r : nullptr;
+  if (!lk.owns_lock()) return nullptr;
+  if (ensure_ring(*r) == cudaSuccess) return r;
+  cudaGetLastError();
+  return nullptr;
 }
 
 // device -> host, returns with the copy complete

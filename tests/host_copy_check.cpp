@@ -167,6 +167,26 @@ static int route() {
   return rc;
 }
 
+// The slots cannot be had: copies of every size take the direct path, and the
+// slots again once they can
+static int no_pinned_memory() {
+  const size_t n = (size_t(40) << 20) + 8;
+  const Bytes a = pattern(n, 3);
+  Bytes dev(n), back(n);
+  int rc = 0;
+  ring_attach(0);
+  for (bool fail : {true, false, true}) {
+    g_fail_pinned = fail;
+    std::fill(dev.begin(), dev.end(), 0);
+    std::fill(back.begin(), back.end(), 0);
+    rc += verdict(copy_to_device(0, stream(1), dev.data(), a.data(), n) == cudaSuccess, "upload refused");
+    rc += verdict(copy_to_host(0, stream(1), back.data(), dev.data(), n) == cudaSuccess, "download refused");
+    rc += verdict(dev == a && back == a, "wrong bytes");
+  }
+  ring_detach(0);
+  return rc + verdict(g_pinned_live == 0, "pinned slots kept");
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   const size_t MB = size_t(1) << 20;
@@ -177,6 +197,7 @@ int main(int argc, char** argv) {
     return rc;
   }
   if (what == "route") return route();
+  if (what == "no_pinned_memory") return no_pinned_memory();
   std::printf("unknown check\n");
   return 2;
 }
