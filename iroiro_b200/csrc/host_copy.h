@@ -192,10 +192,12 @@ inline cudaError_t ring_copy(int device, cudaStream_t st, CopyRing& ring, bool t
 }
 
 // the ring, locked, if this copy goes through it (not when its slots cannot be
-// allocated: the direct copy needs no pinned memory)
-inline CopyRing* ring_for(int device, bool to_host, const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
+// allocated: the direct copy needs no pinned memory; nor on cudaStreamPerThread,
+// which would be another stream in each of the copy's threads)
+inline CopyRing* ring_for(int device, cudaStream_t st, bool to_host, const void* host, size_t bytes,
+                          std::unique_lock<std::mutex>& lk) {
   CopyRing* r = ring_of(device);
-  if (!r || !ring_pays(to_host, host, bytes) || !host_pageable(host)) return nullptr;
+  if (!r || st == cudaStreamPerThread || !ring_pays(to_host, host, bytes) || !host_pageable(host)) return nullptr;
   lk = std::unique_lock<std::mutex>(r->use, std::try_to_lock);
   if (!lk.owns_lock()) return nullptr;
   if (ensure_ring(*r) == cudaSuccess) return r;
@@ -206,7 +208,7 @@ inline CopyRing* ring_for(int device, bool to_host, const void* host, size_t byt
 // device -> host, returns with the copy complete
 inline cudaError_t copy_to_host(int device, cudaStream_t st, void* host, const void* dev, size_t bytes) {
   std::unique_lock<std::mutex> lk;
-  if (CopyRing* r = ring_for(device, true, host, bytes, lk))
+  if (CopyRing* r = ring_for(device, st, true, host, bytes, lk))
     return ring_copy(device, st, *r, true, static_cast<char*>(host), const_cast<char*>(static_cast<const char*>(dev)),
                      bytes);
   const cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
@@ -217,7 +219,7 @@ inline cudaError_t copy_to_host(int device, cudaStream_t st, void* host, const v
 // reused once this returns)
 inline cudaError_t copy_to_device(int device, cudaStream_t st, void* dev, const void* host, size_t bytes) {
   std::unique_lock<std::mutex> lk;
-  if (CopyRing* r = ring_for(device, false, host, bytes, lk))
+  if (CopyRing* r = ring_for(device, st, false, host, bytes, lk))
     return ring_copy(device, st, *r, false, const_cast<char*>(static_cast<const char*>(host)), static_cast<char*>(dev),
                      bytes);
   return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);

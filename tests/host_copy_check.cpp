@@ -30,6 +30,12 @@ std::map<cudaStream_t, Stream> g_streams;
 bool g_fail_pinned = false;
 int g_pinned_live = 0, g_copies = 0;
 
+// every thread has its own cudaStreamPerThread
+Stream& stream_of(cudaStream_t st) {
+  static thread_local char mine;
+  return g_streams[st == cudaStreamPerThread ? reinterpret_cast<cudaStream_t>(&mine) : st];
+}
+
 void run_until(Stream& s, size_t at) {
   while (s.done < at) {
     std::memcpy(s.queue.front().dst, s.queue.front().src, s.queue.front().bytes);
@@ -68,7 +74,7 @@ cudaError_t cudaEventDestroy(cudaEvent_t e) {
 }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t st) {
   std::lock_guard<std::mutex> lk(g_mutex);
-  Stream& s = g_streams[st];
+  Stream& s = stream_of(st);
   *reinterpret_cast<Event*>(e) = Event{&s, s.queued};
   return cudaSuccess;
 }
@@ -80,7 +86,7 @@ cudaError_t cudaEventSynchronize(cudaEvent_t e) {
 }
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t bytes, cudaMemcpyKind, cudaStream_t st) {
   std::lock_guard<std::mutex> lk(g_mutex);
-  Stream& s = g_streams[st];
+  Stream& s = stream_of(st);
   s.queue.push_back(Op{dst, src, bytes});
   ++s.queued;
   ++g_copies;
@@ -88,7 +94,7 @@ cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t bytes, cudaMemcpy
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t st) {
   std::lock_guard<std::mutex> lk(g_mutex);
-  Stream& s = g_streams[st];
+  Stream& s = stream_of(st);
   run_until(s, s.queued);
   return cudaSuccess;
 }
@@ -187,6 +193,24 @@ static int no_pinned_memory() {
   return rc + verdict(g_pinned_live == 0, "pinned slots kept");
 }
 
+// A context on cudaStreamPerThread, a handle that means another stream in each
+// thread: copies stay in order with the calling thread's work
+static int per_thread_stream() {
+  const size_t n = size_t(40) << 20;
+  const Bytes a = pattern(n, 4), b = pattern(n, 5);
+  Bytes dev(n), other(n), back(n);
+  ring_attach(0);
+  cudaMemcpyAsync(dev.data(), a.data(), n, cudaMemcpyDeviceToDevice, cudaStreamPerThread);
+  copy_to_host(0, cudaStreamPerThread, back.data(), dev.data(), n);
+  int rc = verdict(back == a, "the download overtook the work before it");
+  cudaMemcpyAsync(other.data(), dev.data(), n, cudaMemcpyDeviceToDevice, cudaStreamPerThread);
+  copy_to_device(0, cudaStreamPerThread, dev.data(), b.data(), n);
+  cudaStreamSynchronize(cudaStreamPerThread);
+  rc += verdict(other == a && dev == b, "the upload overtook the work before it");
+  ring_detach(0);
+  return rc;
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   const size_t MB = size_t(1) << 20;
@@ -197,6 +221,7 @@ int main(int argc, char** argv) {
     return rc;
   }
   if (what == "route") return route();
+  if (what == "per_thread_stream") return per_thread_stream();
   if (what == "no_pinned_memory") return no_pinned_memory();
   std::printf("unknown check\n");
   return 2;

@@ -23,12 +23,13 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["other_context", "route", "no_pinned_memory"])
+@pytest.mark.parametrize("what", ["other_context", "route", "no_pinned_memory", "per_thread_stream"])
 def test_host_copy(check, what):
     """other_context: an upload on one context's stream, with DMAs still
     queued, then copies of another context of the same device.
     route: the sizes from which a copy goes through the slots, by direction and
     by whether the destination was touched before.
-    no_pinned_memory: the allocation of the slots fails; the copies go on."""
+    no_pinned_memory: the allocation of the slots fails; the copies go on.
+    per_thread_stream: a context on cudaStreamPerThread."""
     r = subprocess.run([str(check), what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
