@@ -440,6 +440,10 @@ struct PtcLayer {
   static constexpr bool AHEAD = CIN >= 8;
   static constexpr int THREADS = NT == 1 && CIN < 16 ? 512 : NT == 4 && CIN >= 8 ? 256 : 384;
   static constexpr int SMEM = WORDS * 4 + (THREADS / 32) * A_BYTES;
+  // four warps sharing a tile's displacements (a few tiles per SM): the tiles of
+  // a CTA, and the bytes of each one's partial sums
+  static constexpr int SLOTS = RAW ? 0 : THREADS / 128;
+  static constexpr int RED_BYTES = 4 * 6 * NT * 32 * 16;
 };
 
 // The channels of displacement D at one site, transported, as BF16 rows of the
@@ -605,10 +609,12 @@ __device__ __forceinline__ void layer_dir(const PtcGeo& G, const float2* __restr
   }
 }
 
-template <int CIN, int COUT>
+// PARTS 4: four warps share a tile, one pair of directions each, the first also
+// the site itself
+template <int CIN, int COUT, int PARTS>
 __global__ void __launch_bounds__(PtcLayer<CIN, COUT>::THREADS, 1)
     ptc_layer_kernel(PtcGeo G, const float2* __restrict__ in, float2* __restrict__ out,
-                     const __nv_bfloat16* __restrict__ bop, int ntiles) {
+                     const __nv_bfloat16* __restrict__ bop, int ntiles, int slots) {
   if (G.skip && *G.skip) return;
   using S = PtcLayer<CIN, COUT>;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -619,7 +625,10 @@ __global__ void __launch_bounds__(PtcLayer<CIN, COUT>::THREADS, 1)
   // (displacement d, channel block h, tile n) holds two consecutive k of
   // output row 8n + l/4
   constexpr int KP = Ptc<CIN, COUT>::KP;
-  for (int i = threadIdx.x; i < S::WORDS; i += S::THREADS) {
+#pragma unroll
+  for (int j = 0; j < (S::WORDS + S::THREADS - 1) / S::THREADS; ++j) {
+    const int i = threadIdx.x + j * S::THREADS;
+    if (i >= S::WORDS) break;
     const int l = i & 31, k = (i >> 5) % S::NB, n = (i >> 5) / S::NB % S::NT;
     const int dh = (i >> 5) / (S::NB * S::NT), d = dh / S::NH, h = dh % S::NH;
     const int part = S::CH == 8 ? k : (l & 3) >> 1;
@@ -630,8 +639,9 @@ __global__ void __launch_bounds__(PtcLayer<CIN, COUT>::THREADS, 1)
   const int lj = lane >> 3, lr = lane & 7;
   const uint32_t a_addr = smem_u32(As) + (S::CH == 4 ? uint32_t((8 * lj + lr) * S::AS)
                                                      : uint32_t((8 * (lj & 1) + lr) * S::AS + 16 * (lj >> 1)));
-  constexpr int NW = S::THREADS / 32;
-  for (int tile = blockIdx.x * NW + warp; tile < ntiles; tile += gridDim.x * NW) {
+  const int slot = warp / PARTS, part = warp % PARTS;
+  if (slot >= slots) return;
+  for (int tile = blockIdx.x * slots + slot; tile < ntiles; tile += gridDim.x * slots) {
     const int p = tile & 1, hs = (tile >> 1) * kFwdSites + lane;
     const Coord c = coord_of(G.g, hs, p);
     int nb[8];
@@ -656,16 +666,47 @@ __global__ void __launch_bounds__(PtcLayer<CIN, COUT>::THREADS, 1)
         mul_dir4<COUT, 2>(ra, 2 * mu + 2, W, As, a_addr, acc);
       }
     } else {
-      if constexpr (S::AHEAD) prefetch_dir<CIN, 1>(G, in, p, hs, 0, nb[0]);
-      layer_dir<CIN, COUT, 0>(G, in, p, hs, 0, 0, W, As, a_addr, acc);
+      const int m0 = part, m1 = PARTS > 1 ? part + 1 : 4;
+      if constexpr (S::AHEAD)
+        prefetch_dir<CIN, 1>(G, in, p, hs, m0, m0 == 0 ? nb[0] : m0 == 1 ? nb[2] : m0 == 2 ? nb[4] : nb[6]);
+      if (part == 0) layer_dir<CIN, COUT, 0>(G, in, p, hs, 0, 0, W, As, a_addr, acc);
 #pragma unroll 1
-      for (int mu = 0; mu < 4; ++mu) {
+      for (int mu = m0; mu < m1; ++mu) {
         const int nf = mu == 0 ? nb[0] : mu == 1 ? nb[2] : mu == 2 ? nb[4] : nb[6];
         const int nr = mu == 0 ? nb[1] : mu == 1 ? nb[3] : mu == 2 ? nb[5] : nb[7];
         if constexpr (S::AHEAD) prefetch_dir<CIN, 2>(G, in, p, hs, mu, nr);
         layer_dir<CIN, COUT, 1>(G, in, p, hs, mu, nf, W, As, a_addr, acc);
-        if (S::AHEAD && mu < 3) prefetch_dir<CIN, 1>(G, in, p, hs, mu + 1, mu == 0 ? nb[2] : mu == 1 ? nb[4] : nb[6]);
+        if (S::AHEAD && mu + 1 < m1)
+          prefetch_dir<CIN, 1>(G, in, p, hs, mu + 1, mu == 0 ? nb[2] : mu == 1 ? nb[4] : nb[6]);
         layer_dir<CIN, COUT, 2>(G, in, p, hs, mu, nr, W, As, a_addr, acc);
+      }
+      if constexpr (PARTS > 1) {
+        // the four warps' sums, each warp adding one column tile in order
+        float4* red = reinterpret_cast<float4*>(smem + S::SMEM + slot * S::RED_BYTES);
+#pragma unroll
+        for (int m = 0; m < 6; ++m)
+#pragma unroll
+          for (int n = 0; n < S::NT; ++n)
+            red[((part * 6 + m) * S::NT + n) * 32 + lane] =
+                make_float4(acc[m][n][0], acc[m][n][1], acc[m][n][2], acc[m][n][3]);
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + slot) : "memory");
+#pragma unroll
+        for (int n = 0; n < S::NT; ++n)
+          if (n == part)
+#pragma unroll
+            for (int m = 0; m < 6; ++m) {
+              float4 v = red[(m * S::NT + n) * 32 + lane];
+#pragma unroll
+              for (int k = 1; k < 4; ++k) {
+                const float4 w = red[((k * 6 + m) * S::NT + n) * 32 + lane];
+                v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+              }
+              acc[m][n][0] = v.x;
+              acc[m][n][1] = v.y;
+              acc[m][n][2] = v.z;
+              acc[m][n][3] = v.w;
+            }
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + slot) : "memory");  // read before the next tile's
       }
     }
     // Lane (g, t) = (lane / 4, lane % 4) holds channel 4n + t of rows g and
@@ -678,6 +719,7 @@ __global__ void __launch_bounds__(PtcLayer<CIN, COUT>::THREADS, 1)
     for (int m = 0; m < 6; ++m)
 #pragma unroll
       for (int n = 0; n < S::NT; ++n) {
+        if (PARTS > 1 && n != part) continue;
         const float* v = acc[m][n];
         const float r0 = __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[2], 1);
         const float r1 = __shfl_xor_sync(0xffffffffu, odd ? v[1] : v[3], 1);
@@ -700,22 +742,38 @@ static int sm_count() {
   return n;
 }
 
-template <int CIN, int COUT>
-static cudaError_t fwd_t(const PtcGeo& G, const float2* in, float2* out, const __nv_bfloat16* bop,
-                         cudaStream_t st) {
+template <int CIN, int COUT, int PARTS>
+static cudaError_t fwd_go(const PtcGeo& G, const float2* in, float2* out, const __nv_bfloat16* bop, int ntiles,
+                          int slots, cudaStream_t st) {
   using S = PtcLayer<CIN, COUT>;
+  constexpr int SMEM = S::SMEM + (PARTS > 1 ? S::SLOTS * S::RED_BYTES : 0);
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(ptc_layer_kernel<CIN, COUT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(ptc_layer_kernel<CIN, COUT, PARTS>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  // one CTA per SM (its register budget), each warp looping over tiles
-  const int ntiles = (G.V + kFwdSites - 1) / kFwdSites;
-  const int grid = std::min((ntiles + S::THREADS / 32 - 1) / (S::THREADS / 32), sm_count());
-  ptc_layer_kernel<CIN, COUT><<<grid, S::THREADS, S::SMEM, st>>>(G, in, out, bop, ntiles);
+  const int grid = std::min((ntiles + slots - 1) / slots, sm_count());
+  ptc_layer_kernel<CIN, COUT, PARTS><<<grid, S::THREADS, SMEM, st>>>(G, in, out, bop, ntiles, slots);
   return cudaGetLastError();
+}
+
+// One CTA per SM (its register budget), each warp looping over tiles;
+// consecutive tiles in one CTA, which share the lines of their gathers.  A small
+// lattice's tiles are spread over all SMs, and while four warps per tile fit,
+// those share its displacements (not with 4 channels in and few out, where a
+// lone warp is fast enough).  An application in full CTAs / spread / shared too,
+// us: (4,4,4,4) 2^12 sites 53 / 41, (4,8,8,4) 2^11 64 / 48 / 38, (4,16,16,16,4)
+// 2^12 107 / 82 / 54, 2^13 - / 83 / 59, 2^14 (two layers shared) 116 / 88 / 90.
+template <int CIN, int COUT>
+static cudaError_t fwd_t(const PtcGeo& G, const float2* in, float2* out, const __nv_bfloat16* bop, cudaStream_t st) {
+  using S = PtcLayer<CIN, COUT>;
+  const int ntiles = (G.V + kFwdSites - 1) / kFwdSites;
+  const int per_sm = (ntiles + sm_count() - 1) / sm_count();
+  if constexpr (S::SLOTS > 0)
+    if (per_sm <= S::SLOTS) return fwd_go<CIN, COUT, 4>(G, in, out, bop, ntiles, per_sm, st);
+  return fwd_go<CIN, COUT, 1>(G, in, out, bop, ntiles, std::min(per_sm, S::THREADS / 32), st);
 }
 
 // CTAs of the weight-gradient kernel (its partial buffer holds as many)

@@ -40,6 +40,24 @@ def test_forward_vs_oracle(small, widths):
     assert rel(got, want) < TOL_NET
 
 
+@pytest.mark.parametrize("L", [[2, 4, 4, 2], [8, 8, 8, 10], [8, 8, 12, 16], [8, 8, 16, 18], [8, 16, 16, 20]])
+@pytest.mark.parametrize("widths", [(4, 4), (4, 16, 16, 4), (4, 8, 16, 8, 4)])
+def test_forward_over_small_lattices(L, widths):
+    """Two, 160, 384, 576 and 1280 tiles of 32 sites: one to several tiles per
+    SM, where a tile is shared by four warps or belongs to one, the last CTA
+    not full."""
+    V = int(np.prod(L))
+    u = ib.synth_gauge(L, 0.25, 25, gauge_transform=True)
+    ctx = ib.Context(L, 0)
+    ctx.upload_gauge(u, force=True)
+    Ws = learned.init_weights(widths, seed=7, scale=0.5)
+    f = ib.synth_gaussian(V, 33)
+    got = learned.PTCNet(ctx, widths, Ws).apply(f)
+    lat = ptc.Lattice(L, u)
+    want = ptc.feat_to_spinor(lat, ptc.forward(lat, Ws, ptc.spinor_to_feat(lat, f))[-1])
+    assert rel(got, want) < TOL_NET
+
+
 def test_loss_and_gradients_vs_oracle(small):
     L, u, ctx = small
     V = int(np.prod(L))
