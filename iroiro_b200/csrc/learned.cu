@@ -26,9 +26,8 @@
 //
 // Backward: the gradient of the input is a layer of the same kind on dY, with
 // adjoint weights and the displacements reversed (T_{+mu}^dag = T_{-mu}), so it
-// runs in the forward kernels; dB = A^T dY accumulates in registers over a
-// CTA's tiles on the tensor cores (mma.sync, the FP32 dY split into three
-// BF16 terms), with a deterministic reduction over the CTAs.
+// runs in the forward kernels; dB = A^T dY is summed in FP32 over a tile and in
+// FP64 over the tiles, with a deterministic reduction over the CTAs.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -197,20 +196,6 @@ __device__ __forceinline__ int fwd_tile_site0(const PtcGeo& G, int tile) {
 constexpr int kDbThreads = 288;
 
 // ---- backward: dB[n][k] = sum over rows (site, colour) of dY[row][n] A[row][k] ------
-// ldmatrix, four 8x8 BF16 matrices transposed: lane l gives the address of row
-// l % 8 of matrix l / 8
-__device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t r[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr)
-               : "memory");
-}
-__device__ __forceinline__ void ldsm2_t(uint32_t addr, uint32_t r[2]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
-               : "=r"(r[0]), "=r"(r[1])
-               : "r"(addr)
-               : "memory");
-}
 // c (16x8, FP32) += a (16x16) b (16x8), BF16
 __device__ __forceinline__ void mma_16816(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -222,166 +207,155 @@ __device__ __forceinline__ void mma_16816(float c[4], const uint32_t a[4], uint3
 
 // Weight gradient of a layer.  Persistent CTAs of 9 warps loop over tiles of
 // 32 sites.  Warp d transports the tile's input channels along displacement d
-// (as the forward kernel) and multiplies its own 2*CIN columns of A with the
-// tile's dY: per colour, the 32 sites are the contraction index of two
-// m16n8k16 steps, M = the layer's real outputs, N = the warp's columns.  dY
-// stays FP32 in value: it is staged as three BF16 terms (hi + mid + lo, 24
-// bits), each multiplied with A and summed in FP32.  The accumulators live in
-// registers over all of a CTA's tiles, so a CTA writes one partial of dB; the
-// sum over CTAs is in block order.
+// (as the forward kernel, rounded to BF16) and multiplies its own 2*CIN columns
+// of A with the tile's FP32 dY: per colour the 32 sites are the contraction
+// index, and lane (ng, kg) holds a TN x TK block of the sum in registers, its
+// operands read from shared memory.
 //
-// What bounds it is the transport (the gathers), as in the forward kernel;
-// the contraction takes 144 MMAs a warp and tile.  Before, each 42-site tile
-// was multiplied on the CUDA cores from shared memory and wrote its own
-// partial.  A 16->16 layer at 16^3x32: 2.33 ms before, 0.147 ms
-// now (and the input gradient, a product stored as FP32 rows and gathered back,
-// 2.30 ms, is a 0.109 ms forward layer).
+// The sum of a tile (96 rows) is FP32 with FMAs; tiles are added in FP64, in
+// the CTA's own block of `partial`, in the order of the tiles, and the CTAs in
+// block order.  The tensor cores take the same products at a quarter of the
+// time, but truncate their FP32 sums: their error was one-sided and grew with
+// the volume, on unit links against a 64-bit sum of the same operands 2.6e-7 at
+// 8^3x16, 3.4e-6 at 16^3x32, 1.7e-5 at 24^3x48, against 3.3e-8 (the result's own rounding) here at all three.
+//
+// Bound by the FMAs and their operand loads.  A training step of
+// (4,16,16,16,4) at 16^3x32 takes 1.51 ms with it, 1.19 ms on the tensor cores.
 template <int CIN, int COUT>
 struct PtcDb {
   static constexpr int NF = 2 * COUT;
-  static constexpr int MT = (NF + 15) / 16;      // 16-row output tiles
   static constexpr int CH = CIN < 8 ? CIN : 8;    // channels transported at a time (registers)
   static constexpr int NH = CIN / CH;
   static constexpr int KC = 2 * CH;               // columns staged at a time: re, then im
-  static constexpr int NT = KC / 8;               // their 8-column tiles
-  static constexpr int YS = MT * 32 + 16;         // bytes of a dY row (padded: conflict-free ldmatrix)
-  static constexpr int AS = NT == 1 ? 16 : 48;    // bytes of an A row (as above)
-  static constexpr int Y_BYTES = 96 * YS;         // one split of one tile
+  static constexpr int TN = NF * KC >= 128 ? 4 : 2;
+  static constexpr int TK = NF * KC / (32 * TN);
+  static constexpr int NG = NF / TN;              // lane = kg * NG + ng
+  static constexpr int NACC = NH * TN * TK;       // entries of a lane over all columns
+  static constexpr int YS = NF * 4 + 16;          // bytes of a dY row (padded: conflict-free)
+  static constexpr int AS = KC * 4 + 16;          // bytes of an A row (as above)
+  static constexpr int Y_BYTES = 96 * YS;
   static constexpr int A_BYTES = 32 * AS;         // one colour of one warp
-  static constexpr int SMEM = 2 * 3 * Y_BYTES + 9 * A_BYTES;
+  static constexpr int SMEM = 2 * Y_BYTES + 9 * A_BYTES;
 };
+
+// N consecutive floats of shared memory
+template <int N>
+__device__ __forceinline__ void lds(const unsigned char* p, float v[N]) {
+  if constexpr (N == 4) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x;
+    v[1] = x.y;
+    v[2] = x.z;
+    v[3] = x.w;
+  } else if constexpr (N == 2) {
+    const float2 x = *reinterpret_cast<const float2*>(p);
+    v[0] = x.x;
+    v[1] = x.y;
+  } else {
+    v[0] = *reinterpret_cast<const float*>(p);
+  }
+}
+__device__ __forceinline__ float2 bf16_pair(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kDbThreads, 2) ptc_db_kernel(PtcGeo G, const float2* __restrict__ in,
                                                              const float2* __restrict__ dy,
-                                                             float* __restrict__ partial, int ntiles) {
+                                                             double* __restrict__ partial, int ntiles) {
   using S = PtcDb<CIN, COUT>;
   constexpr int NW = S::CH / 2;
   extern __shared__ __align__(1024) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char* As = smem + 6 * S::Y_BYTES + warp * S::A_BYTES;
-  // the padding columns of dY (COUT = 4: 8 of 16) stay zero
-  for (int b = threadIdx.x * 16; b < 6 * S::Y_BYTES; b += kDbThreads * 16)
-    *reinterpret_cast<uint4*>(smem + b) = make_uint4(0, 0, 0, 0);
-  __syncthreads();
-  float acc[S::MT][S::NH * S::NT][4];
-#pragma unroll
-  for (int m = 0; m < S::MT; ++m)
-#pragma unroll
-    for (int n = 0; n < S::NH * S::NT; ++n)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc[m][n][k] = 0.f;
-  // ldmatrix addresses of this lane: matrix j = lane / 8 of dY covers rows
-  // 8 (j / 2) and columns 8 (j % 2), of A rows 8 (j % 2) and columns 8 (j / 2)
-  const int lj = lane >> 3, lr = lane & 7;
-  const uint32_t y_off = uint32_t((8 * (lj >> 1) + lr) * S::YS + 16 * (lj & 1));
-  const uint32_t a_off = smem_u32(As) + uint32_t((8 * (lj & 1) + lr) * S::AS + 16 * (lj >> 1));
+  const int ng = lane % S::NG, kg = lane / S::NG;
+  unsigned char* As = smem + 2 * S::Y_BYTES + warp * S::A_BYTES;
+  double* sums = partial + (size_t(blockIdx.x) * 9 + warp) * S::NACC * 32 + lane;
   for (int tile = blockIdx.x, it = 0; tile < ntiles; tile += gridDim.x, ++it) {
     const int site0 = fwd_tile_site0(G, tile);
-    unsigned char* Y = smem + (it & 1) * 3 * S::Y_BYTES;
+    unsigned char* Y = smem + (it & 1) * S::Y_BYTES;
     // dY of the tile: float4 row (3q + colour) of 32 sites -> columns 4q .. 4q+3
     // (re 2q, re 2q+1, im 2q, im 2q+1) of rows 32 colour + site
     for (int j = threadIdx.x; j < 32 * 3 * (COUT / 2); j += kDbThreads) {
       const int sl = j & 31, qa = j >> 5;
       const int q = qa / 3, a = qa - 3 * q;
-      const float4 v = __ldg(reinterpret_cast<const float4*>(dy) + size_t(qa) * G.V + site0 + sl);
-      float x[4] = {v.x, v.y, v.z, v.w};
-      unsigned char* row = Y + (32 * a + sl) * S::YS + 8 * q;
-#pragma unroll
-      for (int sp = 0; sp < 3; ++sp) {
-        const __nv_bfloat162 b01 = __floats2bfloat162_rn(x[0], x[1]);
-        const __nv_bfloat162 b23 = __floats2bfloat162_rn(x[2], x[3]);
-        *reinterpret_cast<uint2*>(row + sp * S::Y_BYTES) = make_uint2(
-            *reinterpret_cast<const uint32_t*>(&b01), *reinterpret_cast<const uint32_t*>(&b23));
-        const float2 f01 = __bfloat1622float2(b01), f23 = __bfloat1622float2(b23);
-        x[0] -= f01.x;
-        x[1] -= f01.y;
-        x[2] -= f23.x;
-        x[3] -= f23.y;
-      }
+      *reinterpret_cast<float4*>(Y + (32 * a + sl) * S::YS + 16 * q) =
+          __ldg(reinterpret_cast<const float4*>(dy) + size_t(qa) * G.V + site0 + sl);
     }
-    const uint32_t y0 = smem_u32(Y) + y_off;
-#pragma unroll
+#pragma unroll 1
     for (int h = 0; h < S::NH; ++h) {
       uint32_t wre[3][NW], wim[3][NW];
       transport_words<S::CH>(G, in + size_t(24 * h) * G.V, site0 + lane, warp, wre, wim);
       // one barrier a tile: the other dY buffer is written next, and this one
       // again only after every warp has passed the next tile's barrier
       if (h == 0) __syncthreads();
+      float acc[S::TN][S::TK];
+#pragma unroll
+      for (int n = 0; n < S::TN; ++n)
+#pragma unroll
+        for (int k = 0; k < S::TK; ++k) acc[n][k] = 0.f;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         __syncwarp();
         unsigned char* row = As + lane * S::AS;
-        if constexpr (CIN == 4) {
-          *reinterpret_cast<uint4*>(row) = make_uint4(wre[a][0], wre[a][1], wim[a][0], wim[a][1]);
-        } else {
-          *reinterpret_cast<uint4*>(row) = make_uint4(wre[a][0], wre[a][1], wre[a][2], wre[a][3]);
-          *reinterpret_cast<uint4*>(row + 16) = make_uint4(wim[a][0], wim[a][1], wim[a][2], wim[a][3]);
+#pragma unroll
+        for (int q = 0; q < NW; q += 2) {
+          const float2 r0 = bf16_pair(wre[a][q]), r1 = bf16_pair(wre[a][q + 1]);
+          const float2 i0 = bf16_pair(wim[a][q]), i1 = bf16_pair(wim[a][q + 1]);
+          *reinterpret_cast<float4*>(row + 8 * q) = make_float4(r0.x, r0.y, r1.x, r1.y);
+          *reinterpret_cast<float4*>(row + 4 * S::CH + 8 * q) = make_float4(i0.x, i0.y, i1.x, i1.y);
         }
         __syncwarp();
+        const unsigned char* yp = Y + 32 * a * S::YS + 4 * S::TN * ng;
+        const unsigned char* ap = As + 4 * S::TK * kg;
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r) {
+          float yv[S::TN], av[S::TK];
+          lds<S::TN>(yp + r * S::YS, yv);
+          lds<S::TK>(ap + r * S::AS, av);
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-          uint32_t b[4];
-          if constexpr (S::NT == 1)
-            ldsm2_t(a_off + uint32_t(16 * ks * S::AS), b);
-          else
-            ldsm4_t(a_off + uint32_t(16 * ks * S::AS), b);
+          for (int n = 0; n < S::TN; ++n)
 #pragma unroll
-          for (int m = 0; m < S::MT; ++m)
-#pragma unroll
-            for (int sp = 2; sp >= 0; --sp) {
-              uint32_t ya[4];
-              ldsm4_t(y0 + uint32_t(sp * S::Y_BYTES + (32 * a + 16 * ks) * S::YS + 32 * m), ya);
-#pragma unroll
-              for (int n = 0; n < S::NT; ++n)
-                mma_16816(acc[m][h * S::NT + n], ya, b[2 * n], b[2 * n + 1]);
-            }
+            for (int k = 0; k < S::TK; ++k) acc[n][k] += yv[n] * av[k];
         }
       }
+      double* p = sums + size_t(h) * S::TN * S::TK * 32;
+#pragma unroll
+      for (int n = 0; n < S::TN; ++n)
+#pragma unroll
+        for (int k = 0; k < S::TK; ++k) {
+          double* e = p + (n * S::TK + k) * 32;
+          *e = it == 0 ? double(acc[n][k]) : *e + double(acc[n][k]);
+        }
     }
   }
-  // row n' = 4q + j of the accumulators is output n = 2o + re/im with
-  // o = 2q + (j & 1), re/im = j >> 1; the columns of tile (h, t) are the real
-  // (t = 0) or imaginary (t = 1) parts of channels 8h .. 8h + 7 (4 input
-  // channels: one tile, re then im), k = (2d + re/im) CIN + channel
-  constexpr int KF = 18 * CIN;
-  float* out = partial + size_t(blockIdx.x) * S::NF * KF + warp * 2 * CIN + 2 * (lane & 3);
-#pragma unroll
-  for (int m = 0; m < S::MT; ++m)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int np = 16 * m + 8 * h + (lane >> 2);
-      if (np < S::NF) {
-        const int n = 2 * (2 * (np >> 2) + (np & 1)) + ((np >> 1) & 1);
-#pragma unroll
-        for (int t = 0; t < S::NH * S::NT; ++t)
-          *reinterpret_cast<float2*>(out + size_t(n) * KF + (t % S::NT) * CIN + 8 * (t / S::NT)) =
-              make_float2(acc[m][t][2 * h], acc[m][t][2 * h + 1]);
-      }
-    }
 }
 
-// Deterministic sum over the CTAs' partials: 8 threads take every 8th partial
-// of one entry, and their sums are added in order (one thread per entry kept
-// 36 blocks busy with a serial chain of loads over one partial per tile: 374 us
-// a call, 6 us now).
+// Deterministic sum over the CTAs' blocks of sums: 8 threads take every 8th
+// block of one entry, and their sums are added in order.  An entry is (warp,
+// column block h, n, k of the lane's block, lane) of ptc_db_kernel; its place in
+// dB[n][k]: column np = 4q + j of dY is output n = 2o + re/im with o = 2q +
+// (j & 1), re/im = j >> 1; A's column is the real or imaginary part of a channel.
 constexpr int kSumSlices = 8;
-__global__ void __launch_bounds__(32 * kSumSlices) sum_partials_kernel(const float* __restrict__ partial,
-                                                                       int nparts, int n, float* out) {
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(32 * kSumSlices) sum_partials_kernel(const double* __restrict__ partial,
+                                                                       int nparts, float* out) {
+  using S = PtcDb<CIN, COUT>;
+  constexpr int n = 9 * S::NACC * 32;  // a multiple of 32
   __shared__ double sm[kSumSlices][32];
-  const int q = blockIdx.x * 32 + threadIdx.x, sl = threadIdx.y;
+  const int lane = threadIdx.x, q = blockIdx.x * 32 + lane, sl = threadIdx.y;
   double acc = 0.0;
-  if (q < n) {
 #pragma unroll 8
-    for (int t = sl; t < nparts; t += kSumSlices) acc += double(__ldg(partial + size_t(t) * n + q));
-  }
-  sm[sl][threadIdx.x] = acc;
+  for (int t = sl; t < nparts; t += kSumSlices) acc += __ldg(partial + size_t(t) * n + q);
+  sm[sl][lane] = acc;
   __syncthreads();
-  if (sl == 0 && q < n) {
+  if (sl != 0) return;
 #pragma unroll
-    for (int k = 1; k < kSumSlices; ++k) acc += sm[k][threadIdx.x];
-    out[q] = float(acc);
-  }
+  for (int k = 1; k < kSumSlices; ++k) acc += sm[k][lane];
+  const int e = blockIdx.x % S::NACC, d = blockIdx.x / S::NACC;
+  const int h = e / (S::TN * S::TK), tn = e / S::TK % S::TN, tk = e % S::TK;
+  const int np = lane % S::NG * S::TN + tn, col = lane / S::NG * S::TK + tk;
+  const int o = 2 * (np >> 2) + (np & 1), part = (np >> 1) & 1;
+  out[size_t(2 * o + part) * 18 * CIN + (2 * d + col / S::CH) * CIN + S::CH * h + col % S::CH] = float(acc);
 }
 
 // spinor field (FP32, full lattice) <-> 4-channel features [site][spin][colour]
@@ -776,14 +750,14 @@ static cudaError_t fwd_t(const PtcGeo& G, const float2* in, float2* out, const _
   return fwd_go<CIN, COUT, 1>(G, in, out, bop, ntiles, std::min(per_sm, S::THREADS / 32), st);
 }
 
-// CTAs of the weight-gradient kernel (its partial buffer holds as many)
+// CTAs of the weight-gradient kernel (its buffer of sums holds as many blocks)
 static int db_grid(int V) {
   const int ntiles = (V + kFwdSites - 1) / kFwdSites;
   return std::min(ntiles, 2 * sm_count());
 }
 
 template <int CIN, int COUT>
-static cudaError_t db_t(const PtcGeo& G, const float2* in, const float2* dy, float* partial, float* db,
+static cudaError_t db_t(const PtcGeo& G, const float2* in, const float2* dy, double* partial, float* db,
                         cudaStream_t st) {
   using S = PtcDb<CIN, COUT>;
   static bool attr = false;
@@ -798,8 +772,7 @@ static cudaError_t db_t(const PtcGeo& G, const float2* in, const float2* dy, flo
                                                                (G.V + kFwdSites - 1) / kFwdSites);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const int n = S::NF * 18 * CIN;
-  sum_partials_kernel<<<(n + 31) / 32, dim3(32, kSumSlices), 0, st>>>(partial, grid, n, db);
+  sum_partials_kernel<CIN, COUT><<<9 * S::NACC, dim3(32, kSumSlices), 0, st>>>(partial, grid, db);
   return cudaGetLastError();
 }
 
@@ -829,7 +802,7 @@ cudaError_t launch_ptc_fwd(int cin, int cout, const PtcGeo& G, const float2* in,
 }
 
 cudaError_t launch_ptc_db(int cin, int cout, const PtcGeo& G, const float2* in, const float2* dy,
-                          float* partial, float* db, cudaStream_t st) {
+                          double* partial, float* db, cudaStream_t st) {
 #define IRO_B(A, B) db_t<A, B>(G, in, dy, partial, db, st)
   IRO_PTC_DISPATCH(IRO_B)
 #undef IRO_B
@@ -1294,7 +1267,7 @@ struct iro_ptc {
   std::vector<float2*> act;           // act[l]: input of layer l (act[nl]: output)
   float2* g0 = nullptr;               // gradient ping-pong buffers
   float2* g1 = nullptr;
-  float* partial = nullptr;           // weight-gradient partials, one per CTA
+  double* partial = nullptr;          // weight-gradient sums, one block per CTA
   float* db = nullptr;                // every layer's dL/dB, consecutive
   double* lpart = nullptr;
   size_t maxc = 0;
@@ -1452,7 +1425,7 @@ int iro_ptc_create(iro_ctx* c, int nlayers, const int* widths, iro_ptc** out) {
   LCK(cudaMalloc(&n->g0, V * maxc * 3 * sizeof(float2)));
   LCK(cudaMalloc(&n->g1, V * maxc * 3 * sizeof(float2)));
   LCK(cudaMalloc(&n->db, gradn * sizeof(float)));
-  LCK(cudaMalloc(&n->partial, size_t(db_grid(int(V))) * maxnk * sizeof(float)));
+  LCK(cudaMalloc(&n->partial, size_t(db_grid(int(V))) * maxnk * sizeof(double)));
   LCK(cudaMalloc(&n->lpart, sizeof(double) * 2 * loss_blocks()));
   *out = n.release();
   return IRO_OK;

@@ -98,6 +98,44 @@ def test_gradients_of_every_layer_shape(widths):
         assert rel(g, go) < 5e-2  # BF16 operands through every layer and back
 
 
+def _bf16(a):
+    """FP32 values rounded to BF16 (to nearest, ties to even), as FP64."""
+    b = np.ascontiguousarray(a, dtype=np.float32).view(np.uint32)
+    b = (b + 0x7fff + ((b >> 16) & 1)) & np.uint32(0xffff0000)
+    return b.view(np.float32).astype(np.float64)
+
+
+@pytest.mark.parametrize("L", [[8, 8, 8, 16], [16, 16, 16, 32]])
+@pytest.mark.parametrize("mean", [0.0, 1.0])
+def test_weight_gradient_against_64_bit_sums(L, mean):
+    """The weight gradient of a (4,4) layer against a 64-bit sum of the same
+    operands: on unit links the transported inputs are the inputs, rounded to
+    BF16, and dL/dy is formed from the layer's own output.  One and 14 tiles per
+    CTA, terms of both signs and of one.  The result is rounded to FP32 (2^-24 =
+    6e-8 at most); a tile's FP32 sum of 96 products errs by some sqrt(96) / 2
+    roundings of random sign, which average out over the 256 tiles and more
+    (5 x 6e-8 / 16 = 2e-8): 1e-7 in all.  Sums truncated as the tensor cores
+    truncate them err by 2.6e-7 on the small lattice and 3.4e-6 on the large one."""
+    V = int(np.prod(L))
+    u = np.zeros((4, V, 3, 3, 2))
+    u[:, :, range(3), range(3), 0] = 1.0
+    u = u.ravel()
+    ctx = ib.Context(L, 0)
+    ctx.upload_gauge(u, force=True)
+    net = learned.PTCNet(ctx, (4, 4), learned.init_weights((4, 4), seed=3, scale=0.5))
+    f32 = lambda a: a.astype(np.float32).astype(np.float64)
+    x, t = f32(ib.synth_gaussian(V, 51) + mean), f32(ib.synth_gaussian(V, 52) - 3.0 * mean)
+    y = net.apply(x)
+    fields = [ib.DeviceField(ctx, 2, "double").upload(f) for f in (x, t)]
+    _, (got,) = net.loss_grad(ctx, *fields)
+    lat = ptc.Lattice(L, u)
+    dy = np.float32(2.0 / np.sum(t * t)) * (y.astype(np.float32) - t.astype(np.float32))
+    dy = ptc.spinor_to_feat(lat, dy.astype(np.float64))
+    a = ptc.spinor_to_feat(lat, _bf16(x))
+    want = np.stack([np.einsum("soa,sia->oi", dy, lat.transport(a, d).conj(), optimize=True) for d in range(9)])
+    assert rel(got, want) < 1e-7
+
+
 def _pair(L, seed):
     u = ib.synth_gauge(L, 0.2, seed)
     ctx = ib.Context(L, 0)
