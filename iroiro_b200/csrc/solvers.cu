@@ -245,7 +245,8 @@ int cg_double(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* 
     }
     return IRO_OK;
   };
-  if (cg_is_small(op, PREC_DOUBLE, nrhs, vh(c)))
+  // (max_iter 0: no iteration, on either path)
+  if (prm->max_iter > 0 && cg_is_small(op, PREC_DOUBLE, nrhs, vh(c)))
     RC(iterate_small(c, op, mass, P, Q, R, X, prm->max_iter));
   else
     RC(iterate(c, nrhs, prm->max_iter, prm->use_graph != 0, body));

@@ -56,6 +56,20 @@ def test_cg_not_converged_raises(g):
         ib.Solver_CG(1e-20, 5, ib.Fopr_DdagD(D)).solve(np.empty_like(b), b)
 
 
+@pytest.mark.parametrize("L", [[4, 4, 4, 8], [16, 16, 16, 32]])
+def test_cg_without_iterations(L):
+    """max_iter = 0 returns the starting guess x0 = b (solver_CG.cpp:40) and its
+    residual, on lattices of the one-launch iteration and of the launched one."""
+    V = int(np.prod(L))
+    u = ib.synth_gauge(L, 0.2, 341, gauge_transform=True)
+    D = ib.Dirac_Wilson_EvenOdd(0.5 / 0.12 - 4, u, ctx=ib.Context(L, 0))
+    b = ib.synth_gaussian(V // 2, 342)
+    x, outs, rc = ib.Solver_CG(1e-20, 0, ib.Fopr_DdagD(D)).solve_many(b, 1)
+    assert rc == ib.NOT_CONVERGED and np.array_equal(x, b)
+    assert outs[0].Iterations == -1 and outs[0].operator_applies == 2
+    assert abs(outs[0].diff - rel(D.mult_dag(D.mult(b)), b)) < 1e-12 * outs[0].diff
+
+
 @pytest.mark.parametrize("inner", ["double", "single", "half"])
 def test_block_cg_12_rhs(inner):
     """12 point sources at one site solved together, each to 1e-10."""
