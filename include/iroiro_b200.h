@@ -369,12 +369,12 @@ int iro_gcr_solve_field(iro_ctx* ctx, int op, double mass, double csw, const iro
                         const iro_gcr_params* prm, const iro_field* b, iro_field* x,
                         iro_gcr_out* out);
 
-/* Self-test of the device-side bounded waits (no counterpart in the
-   reference): a kernel that waits (the small-lattice CG's grid barrier) does so
-   for at most 1 s and then sets an error flag that the host turns into
-   IRO_TIMEOUT, leaving the context usable.  This runs such a wait on an mbarrier
-   that nothing arrives at, for limit_ms (0 < limit_ms <= 1000), and returns IRO_TIMEOUT
-   with the time it waited in *waited_ms. */
+/* Self-test of the device-side bounded wait (no counterpart in the
+   reference): the small-lattice CG's grid barrier waits for at most 1 s; a wait
+   that runs out sets an error flag, and every block leaves.  This runs that
+   barrier, one block per SM, with one arrival missing for limit_ms
+   (0 < limit_ms <= 1000) and returns IRO_TIMEOUT with the time it waited in
+   *waited_ms; the context stays usable. */
 int iro_selftest_bounded_wait(iro_ctx* ctx, double limit_ms, double* waited_ms);
 
 /* ---- synthetic inputs (host) ---------------------------------------------- */

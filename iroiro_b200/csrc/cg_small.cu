@@ -26,6 +26,15 @@ namespace {
 
 using namespace split;
 
+// The barrier of a cooperative grid: the arrivals counted in `bar`, `blocks` of
+// them (the grid's) awaited each time, for at most limit_ns
+struct GridBarrier {
+  unsigned* bar;
+  int* err;
+  unsigned blocks;
+  uint64_t limit_ns;
+};
+
 struct CgSmallParams {
   Geom g;
   int nrhs, full, clover;
@@ -40,8 +49,7 @@ struct CgSmallParams {
   int* done;
   int max_iter, iters;
   double* partials;
-  unsigned* bar;
-  int* err;
+  GridBarrier wait;
 };
 
 template <typename R>
@@ -113,7 +121,7 @@ __device__ __forceinline__ double hop_phase(const CgSmallParams& P, SmallShared<
   return sum;
 }
 
-__device__ __forceinline__ uint64_t small_ns() {
+__device__ __forceinline__ uint64_t global_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
@@ -126,29 +134,28 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 
 // Waits until every block has arrived `gen` times (the counter only grows
 // within a launch).  The grid is resident as a whole (cooperative launch); the
-// wait is bounded all the same: after a second of global time the block sets
+// wait is bounded all the same: after limit_ns of global time the block sets
 // the error flag and leaves, and so do the others.
-template <typename SM>
-__device__ __noinline__ bool grid_barrier(const CgSmallParams& P, SM& sm, unsigned& gen) {
+__device__ __noinline__ bool grid_barrier(const GridBarrier& B, int& shared_ok, unsigned& gen) {
   ++gen;
   __syncthreads();
   if (threadIdx.x == 0) {
     // the block's writes (ordered before this by the barrier above) are
     // released with the arrival, the others' acquired with the last poll
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(P.bar) : "memory");
-    const unsigned want = gen * gridDim.x;
-    const uint64_t t0 = small_ns();
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(B.bar) : "memory");
+    const unsigned want = gen * B.blocks;
+    const uint64_t t0 = global_ns();
     int ok = 1;
-    for (unsigned it = 0; ld_acquire(P.bar) < want; ++it)
-      if ((it & 255u) == 255u && small_ns() - t0 > 1000000000ull) {
+    for (unsigned it = 0; ld_acquire(B.bar) < want; ++it)
+      if ((it & 255u) == 255u && global_ns() - t0 > B.limit_ns) {
         ok = 0;
-        atomicExch(P.err, 1);
+        atomicExch(B.err, 1);
         break;
       }
-    sm.ok = ok;
+    shared_ok = ok;
   }
   __syncthreads();
-  return sm.ok != 0;
+  return shared_ok != 0;
 }
 
 // This block's partials of a sum per right-hand side (fixed order): one right-hand
@@ -315,19 +322,19 @@ __global__ void __launch_bounds__(kThreads, 2) cg_small_kernel(const __grid_cons
       double v = 0.0;
 #pragma unroll 1
       for (int k = first; k < 2; ++k) {
-        if (k > first && !grid_barrier(P, sm, gen)) return;
+        if (k > first && !grid_barrier(P.wait, sm.ok, gen)) return;
         v = hop_phase<SP>(P, sm, site, k, dag);
       }
       double* part = P.partials + dag * set;
       put_partial(P, sm, part, v);
-      if (!grid_barrier(P, sm, gen)) return;
+      if (!grid_barrier(P.wait, sm.ok, gen)) return;
       take_totals(P, sm, part, dag == 0 ? ST_CG_ALPHA : ST_CG_BETA);
     }
     update_phase<SP>(P, sm);
     bool left = true;
     for (int r = 0; r < P.nrhs; ++r) left = left && sm.done[r] != RUNNING;
     if (left) break;  // the same in every block
-    if (!grid_barrier(P, sm, gen)) return;
+    if (!grid_barrier(P.wait, sm.ok, gen)) return;
   }
   __syncthreads();
   if (blockIdx.x == 0 && t < P.nrhs) {
@@ -336,8 +343,17 @@ __global__ void __launch_bounds__(kThreads, 2) cg_small_kernel(const __grid_cons
   }
 }
 
+// Self-test of the barrier (iro_selftest_bounded_wait): the time of one wait
+__global__ void __launch_bounds__(kThreads) barrier_probe_kernel(GridBarrier B, unsigned long long* waited_ns) {
+  __shared__ int ok;
+  unsigned gen = 0;
+  const uint64_t t0 = global_ns();
+  grid_barrier(B, ok, gen);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *waited_ns = global_ns() - t0;
+}
+
 template <int SP>
-cudaError_t go(const CgSmallParams& P, int sms, cudaStream_t st) {
+cudaError_t go(CgSmallParams P, int sms, cudaStream_t st) {
   int per_sm = 0;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cg_small_kernel<SP>, kThreads, 0);
   if (e != cudaSuccess) return e;
@@ -345,7 +361,8 @@ cudaError_t go(const CgSmallParams& P, int sms, cudaStream_t st) {
   const int groups = (P.full ? 2 : 1) * ((P.g.Vh + S - 1) / S);
   int grid = sms * per_sm;
   if (grid > groups) grid = groups;
-  void* args[] = {const_cast<CgSmallParams*>(&P)};
+  P.wait.blocks += grid;
+  void* args[] = {&P};
   return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(cg_small_kernel<SP>), dim3(grid),
                                      dim3(kThreads), args, 0, st);
 }
@@ -378,8 +395,7 @@ cudaError_t launch_cg_small(const CgSmallLaunch& L, cudaStream_t st) {
   P.max_iter = L.max_iter;
   P.iters = L.iters;
   P.partials = L.partials;
-  P.bar = L.bar;
-  P.err = L.err;
+  P.wait = GridBarrier{L.bar, L.err, unsigned(L.missing), L.limit_ns};
   cudaError_t e = cudaMemsetAsync(L.bar, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
   switch (L.p->prec) {
@@ -387,6 +403,16 @@ cudaError_t launch_cg_small(const CgSmallLaunch& L, cudaStream_t st) {
     case PREC_SINGLE: return go<PREC_SINGLE>(P, L.sms, st);
     default: return go<PREC_HALF>(P, L.sms, st);
   }
+}
+
+cudaError_t launch_barrier_probe(int blocks, int missing, uint64_t limit_ns, unsigned* bar, int* err,
+                                 unsigned long long* waited_ns, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(unsigned), st);
+  if (e != cudaSuccess) return e;
+  GridBarrier B{bar, err, unsigned(blocks + missing), limit_ns};
+  void* args[] = {&B, &waited_ns};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(barrier_probe_kernel), dim3(blocks), dim3(kThreads), args,
+                                     0, st);
 }
 
 }  // namespace iro

@@ -112,8 +112,13 @@ struct CgSmallLaunch {
   double* partials;  // 2 * max(4, nrhs) doubles per block
   unsigned* bar;
   int* err;
+  int missing;        // arrivals awaited beyond the grid's own (0; a self-test's 1)
+  uint64_t limit_ns;  // of a wait at the grid barrier
 };
 cudaError_t launch_cg_small(const CgSmallLaunch& L, cudaStream_t st);
+// one wait of its grid barrier by `blocks` blocks (at most one per SM)
+cudaError_t launch_barrier_probe(int blocks, int missing, uint64_t limit_ns, unsigned* bar, int* err,
+                                 unsigned long long* waited_ns, cudaStream_t st);
 
 // Multishift, vectors in FP64 or FP32 (prec), FP64 scalars:
 // x0 -= beta p0; r += beta (s + sigma0 p0); reduce |r|^2

@@ -40,46 +40,8 @@
 
 namespace iro {
 
-// ---- shared-memory addresses; the bounded mbarrier wait of the self-test -----------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t phase) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(phase)
-      : "memory");
-  return ok != 0;
-}
-
-// A wait on an mbarrier gives up after a limit of global time (or kWaitLimit
-// polls, whichever comes first): the kernel then sets its error flag and
-// leaves, and the host reports IRO_TIMEOUT.
-constexpr int kWaitLimit = 1 << 24;
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Polls the barrier until `phase` completes; false after limit_ns of global
-// time or kWaitLimit polls
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t phase, uint64_t limit_ns) {
-  const uint64_t t0 = global_ns();
-  for (int it = 0; it < kWaitLimit; ++it) {
-    if (mbar_try_wait(bar, phase)) return true;
-    if ((it & 63) == 63 && global_ns() - t0 > limit_ns) return false;
-  }
-  return false;
 }
 
 // K and N of the packed real weights B[n][k]: k = (2d + re/im) CIN + i, n = 2o +
@@ -1112,28 +1074,6 @@ __global__ void gcr_gamma_kernel(GcrState* s) {
   }
 }
 
-// Self-test of the bounded wait (iro_selftest_bounded_wait): one thread waits
-// on an mbarrier that nothing arrives at, gives up after limit_ns, and
-// records the time it waited and the error flag, as the tensor-core kernels
-// do on a wait that runs out.
-__global__ void bounded_wait_probe_kernel(uint64_t limit_ns, int* err, unsigned long long* waited_ns) {
-  __shared__ __align__(8) uint64_t bar;
-  if (threadIdx.x == 0) mbar_init(&bar, 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const uint64_t t0 = global_ns();
-    const bool ok = mbar_wait_bounded(&bar, 0u, limit_ns);
-    *waited_ns = global_ns() - t0;
-    if (!ok) atomicExch(err, 1);
-  }
-}
-
-cudaError_t launch_bounded_wait_probe(uint64_t limit_ns, int* err, unsigned long long* waited_ns,
-                                      cudaStream_t st) {
-  bounded_wait_probe_kernel<<<1, 32, 0, st>>>(limit_ns, err, waited_ns);
-  return cudaGetLastError();
-}
-
 template <int PW, int M>
 static void cdot_go(int64_t n, const CFieldList& w, SpinorPtr t, double* part, int blocks,
                     const int* skip, cudaStream_t st) {
@@ -1711,33 +1651,6 @@ int iro_gcr_solve_field(iro_ctx* c, int op, double mass, double csw, const iro_p
     if (e) return e;
   }
   if (!converged) return set_error(c, IRO_NOT_CONVERGED, "GCR not converged");
-  return IRO_OK;
-}
-
-int iro_selftest_bounded_wait(iro_ctx* c, double limit_ms, double* waited_ms) {
-  if (!c || !waited_ms || !(limit_ms > 0.0) || limit_ms > 1000.0) return IRO_BAD_ARG;
-  LCK(cudaSetDevice(device(c)));
-  cudaStream_t st = stream(c);
-  int* err = nullptr;
-  unsigned long long* ns = nullptr;
-  LCK(cudaMalloc(reinterpret_cast<void**>(&err), sizeof(int)));
-  const cudaError_t e0 = cudaMalloc(reinterpret_cast<void**>(&ns), sizeof(unsigned long long));
-  if (e0 != cudaSuccess) {
-    cudaFree(err);
-    return cuda_error(c, e0, "cudaMalloc");
-  }
-  int herr = 0;
-  unsigned long long hns = 0;
-  cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int), st);
-  if (e == cudaSuccess) e = launch_bounded_wait_probe(uint64_t(limit_ms * 1e6), err, ns, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&hns, ns, sizeof(hns), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(err);
-  cudaFree(ns);
-  if (e != cudaSuccess) return cuda_error(c, e, "bounded-wait self-test");
-  *waited_ms = double(hns) * 1e-6;
-  if (herr) return set_error(c, IRO_TIMEOUT, "bounded wait ran out (self-test)");
   return IRO_OK;
 }
 

@@ -154,6 +154,7 @@ bool cg_is_small(int op, int prec, int nrhs, int64_t half_volume) {
 // paused): the inner loop of cg_double and cg_mixed on a small lattice.  A
 // launch is bounded to kSmallIters iterations (a few ms).
 constexpr int kSmallIters = 256;
+constexpr uint64_t kBarrierLimitNs = 1000000000ull;
 int iterate_small(iro_ctx* c, int op, double mass, const DevField* P, const DevField* Q, const DevField* R,
                   const DevField* X, int max_iter) {
   const bool cl = op == IRO_OP_CLOVER_FULL || op == IRO_OP_CLOVER_SCHUR_EE;
@@ -187,6 +188,7 @@ int iterate_small(iro_ctx* c, int op, double mass, const DevField* P, const DevF
   L.partials = partials(c);
   L.bar = sync_words(c);
   L.err = reinterpret_cast<int*>(sync_words(c) + 1);
+  L.limit_ns = kBarrierLimitNs;
   int* hpin = static_cast<int*>(pinned(c));
   for (int64_t launched = 0;;) {
     CK(launch_cg_small(L, st));
@@ -1282,4 +1284,23 @@ extern "C" int iro_md_force(iro_ctx* c, int op, double mass, double csw, const d
     CK(launch_force(g, U, recon, 0, B->half(1), E->half(0), 1, k, F, st));
   }
   return device_to_host(c, force, F, nF * sizeof(double));
+}
+
+extern "C" int iro_selftest_bounded_wait(iro_ctx* c, double limit_ms, double* waited_ms) {
+  if (!c || !waited_ms || !(limit_ms > 0.0) || limit_ms > 1000.0) return IRO_BAD_ARG;
+  CK(cudaSetDevice(device(c)));
+  cudaStream_t st = stream(c);
+  // the time comes back through the context's reduction scratch
+  auto* ns = reinterpret_cast<unsigned long long*>(partials(c));
+  int* err = reinterpret_cast<int*>(sync_words(c) + 1);
+  int herr = 0;
+  unsigned long long hns = 0;
+  CK(launch_barrier_probe(sm_count(c), 1, uint64_t(limit_ms * 1e6), sync_words(c), err, ns, st));
+  CK(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(&hns, ns, sizeof(hns), cudaMemcpyDeviceToHost, st));
+  CK(cudaMemsetAsync(err, 0, sizeof(int), st));
+  CK(cudaStreamSynchronize(st));
+  *waited_ms = double(hns) * 1e-6;
+  if (herr) return set_error(c, IRO_TIMEOUT, "a grid barrier ran out (self-test)");
+  return IRO_OK;
 }

@@ -1,13 +1,13 @@
-"""The device-side bounded wait of the tensor-core kernels: a wait on an
-mbarrier that nothing arrives at runs out after its time limit, the host
-gets IRO_TIMEOUT, and the context keeps working."""
+"""The device-side bounded wait, the grid barrier of the small-lattice CG: with
+an arrival missing every block leaves after the time limit, the host gets
+IRO_TIMEOUT, and the context keeps working."""
 import ctypes
 
 import numpy as np
 import pytest
 
 import iroiro_b200 as ib
-from conftest import TOL_FP64, load_golden, rel
+from conftest import TOL_FP64, TOL_RES, TOL_SOL, load_golden, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -21,7 +21,12 @@ def test_wait_runs_out_and_context_stays_usable(port):
         rc = c._lib.iro_selftest_bounded_wait(c.h, limit, ctypes.byref(waited))
         assert rc == ib.TIMEOUT
         assert limit <= waited.value < limit + 200.0
-    # the context and the device still work: an operator against the oracle
+    # the context and the device still work: a solve over the same barrier, and
+    # an operator against the oracle
+    D = ib.Dirac_Wilson_EvenOdd(float(g["mass"]), g["u"], ctx=c)
+    x = np.empty_like(g["f_half"])
+    assert ib.Solver_CG(1e-20, 5000, ib.Fopr_DdagD(D)).solve(x, g["f_half"]).diff < TOL_RES
+    assert rel(x, g["cg_wilson_eo_x"]) < TOL_SOL
     m = float(g["mass"])
     f = g["f_half"]
     assert rel(c.apply(ib.OP_WILSON_SCHUR_EE, m, 0.0, 0, f),
