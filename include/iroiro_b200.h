@@ -203,8 +203,13 @@ typedef struct {
                        FP64 residual recomputation, solution and reductions */
   double delta;     /* reliable update when |r| < delta * max |r| since the
                        last update (mixed precision only); <= 0 selects 0.1 */
-  int use_graph;    /* capture the iteration as a CUDA graph */
+  int use_graph;    /* nonzero: capture the launched iteration as a CUDA graph.
+                       Small lattices iterate in one cooperative launch
+                       instead, unless IRO_CG_LAUNCHED is added (or
+                       IRO_HOP_VARIANT asks for a launched stencil) */
 } iro_cg_params;
+
+#define IRO_CG_LAUNCHED 256 /* iro_cg_params.use_graph: the launched iteration on every lattice */
 
 /* Solve (D^dagger D) x = b by CG for the operator `op` (Fopr_DdagD with
    Solver_CG, lib/Fopr/fopr.h:146-153, lib/Solver/solver_CG.cpp:29-160).

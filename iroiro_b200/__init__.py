@@ -562,20 +562,26 @@ class SolverOutput:
 _SOLVER_OPS = (OP_WILSON_FULL, OP_WILSON_SCHUR_EE, OP_CLOVER_FULL, OP_CLOVER_SCHUR_EE)
 
 
+CG_LAUNCHED = 256  # IRO_CG_LAUNCHED
+
+
 class Solver_CG:
     """Solver_CG(prec, MaxIter, Fopr_DdagD(D)) (lib/Solver/solver_CG.hpp:28-31).
 
     ``prec`` is the squared relative residual target (GoalPrecision).
     ``inner`` selects the reference's FP64 CG ("double") or the reliable-update
-    mixed-precision CG with FP32 ("single") or FP16 ("half") inner storage."""
+    mixed-precision CG with FP32 ("single") or FP16 ("half") inner storage.
+    ``launched`` keeps the iteration of launched kernels (captured as a graph
+    with ``use_graph``) on small lattices too, which otherwise iterate in one
+    cooperative launch."""
 
     def __init__(self, prec: float, MaxIter: int, fopr: Fopr_DdagD, inner="double",
-                 delta: float = 0.1, use_graph: bool = True):
+                 delta: float = 0.1, use_graph: bool = True, launched: bool = False):
         if not isinstance(fopr, Fopr_DdagD) or fopr.D.op not in _SOLVER_OPS:
             raise IroError(BAD_ARG, "Solver_CG needs Fopr_DdagD of a full or Schur operator")
         self.fopr = fopr
         self.params = CGParams(float(prec), int(MaxIter), _PREC[inner], float(delta),
-                               int(bool(use_graph)))
+                               int(bool(use_graph)) | (CG_LAUNCHED if launched else 0))
 
     def check_DdagD(self) -> bool:
         return True

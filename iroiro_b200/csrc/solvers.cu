@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -142,7 +143,10 @@ int iterate(iro_ctx* c, int nrhs, int max_iter, bool use_graph, F body) {
 //   FP32 clover:  16^4 e/o 1024 6.17 / 5.53, 16^3x32 2048 8.86 / 10.32
 //   FP16 Wilson:  16^4 e/o 1024 4.96 / 4.69, 12^3x16 e/o 3 rhs 1383 5.44 / 5.83
 //   FP16 clover:  12^3x16 e/o 432 5.26 / 3.86, 16^4 1024 5.61 / 5.87
+// IRO_HOP_VARIANT forces a stencil of the launched iteration, so it keeps that.
 bool cg_is_small(int op, int prec, int nrhs, int64_t half_volume) {
+  static const bool forced = std::getenv("IRO_HOP_VARIANT") != nullptr;
+  if (forced) return false;
   static const int limit[3][2] = {{888, 448}, {1480, 1184}, {1036, 740}};
   const bool cl = op == IRO_OP_CLOVER_FULL || op == IRO_OP_CLOVER_SCHUR_EE;
   const int S = 32 / nrhs;  // sites of a group
@@ -206,6 +210,9 @@ int iterate_small(iro_ctx* c, int op, double mass, const DevField* P, const DevF
   }
 }
 
+bool want_graph(const iro_cg_params* prm) { return (prm->use_graph & ~IRO_CG_LAUNCHED) != 0; }
+bool want_launched(const iro_cg_params* prm) { return (prm->use_graph & IRO_CG_LAUNCHED) != 0; }
+
 // FP64 CG on D^dag D, Solver_CG::solve (lib/Solver/solver_CG.cpp:29-80).
 int cg_double(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* prm,
               const DevField* B, DevField* X, int nrhs, iro_solver_out* out) {
@@ -248,10 +255,10 @@ int cg_double(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* 
     return IRO_OK;
   };
   // (max_iter 0: no iteration, on either path)
-  if (prm->max_iter > 0 && cg_is_small(op, PREC_DOUBLE, nrhs, vh(c)))
+  if (prm->max_iter > 0 && !want_launched(prm) && cg_is_small(op, PREC_DOUBLE, nrhs, vh(c)))
     RC(iterate_small(c, op, mass, P, Q, R, X, prm->max_iter));
   else
-    RC(iterate(c, nrhs, prm->max_iter, prm->use_graph != 0, body));
+    RC(iterate(c, nrhs, prm->max_iter, want_graph(prm), body));
   // true residual |A x - b| / |b| (solver_CG.cpp:69-71)
   RC(apply(c, op, mass, csw, false, *X, *Q, nullptr, 0, nullptr));
   RC(apply(c, op, mass, csw, true, *Q, *S, nullptr, 0, nullptr));
@@ -988,9 +995,9 @@ int cg_mixed(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* p
     }
     return IRO_OK;
   };
-  const bool small = !shifted && cg_is_small(op, pl, nrhs, vh(c));
+  const bool small = !shifted && !want_launched(prm) && cg_is_small(op, pl, nrhs, vh(c));
   cudaGraphExec_t exec = nullptr;
-  if (!small && prm->use_graph && st != nullptr) {
+  if (!small && want_graph(prm) && st != nullptr) {
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int brc = body(kChunk);

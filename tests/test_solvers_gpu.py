@@ -28,9 +28,12 @@ def _dirac(g, name):
 
 @pytest.mark.parametrize("name", ["wilson_full", "wilson_eo", "clover_full"])
 @pytest.mark.parametrize("graph", [False, True])
-def test_cg_fp64_vs_reference(g, name, graph):
+@pytest.mark.parametrize("launched", [True, False])
+def test_cg_fp64_vs_reference(g, name, graph, launched):
+    """The launched iteration with and without a graph, and the one-launch
+    iteration of small lattices."""
     D, b = _dirac(g, name)
-    slv = ib.Solver_CG(1e-20, 5000, ib.Fopr_DdagD(D), use_graph=graph)
+    slv = ib.Solver_CG(1e-20, 5000, ib.Fopr_DdagD(D), use_graph=graph, launched=launched)
     x = np.empty_like(b)
     out = slv.solve(x, b)
     assert abs(out.Iterations - int(g[f"cg_{name}_iters"])) <= 2
@@ -40,9 +43,10 @@ def test_cg_fp64_vs_reference(g, name, graph):
 
 @pytest.mark.parametrize("name", ["wilson_full", "wilson_eo", "clover_full"])
 @pytest.mark.parametrize("inner", ["single", "half"])
-def test_cg_mixed_precision(g, name, inner):
+@pytest.mark.parametrize("launched", [True, False])
+def test_cg_mixed_precision(g, name, inner, launched):
     D, b = _dirac(g, name)
-    slv = ib.Solver_CG(1e-20, 5000, ib.Fopr_DdagD(D), inner=inner)
+    slv = ib.Solver_CG(1e-20, 5000, ib.Fopr_DdagD(D), inner=inner, launched=launched)
     x = np.empty_like(b)
     out = slv.solve(x, b)
     assert out.diff < TOL_RES
@@ -71,8 +75,10 @@ def test_cg_without_iterations(L):
 
 
 @pytest.mark.parametrize("inner", ["double", "single", "half"])
-def test_block_cg_12_rhs(inner):
-    """12 point sources at one site solved together, each to 1e-10."""
+@pytest.mark.parametrize("launched", [True, False])
+def test_block_cg_12_rhs(inner, launched):
+    """12 point sources at one site solved together, each to 1e-10, by the
+    launched iteration (fused r updates and reductions) and by the rule's."""
     L = [8, 8, 8, 8]
     V = int(np.prod(L))
     c = ib.context(L)
@@ -80,7 +86,7 @@ def test_block_cg_12_rhs(inner):
     c.upload_gauge(u, force=True)
     D = ib.Dirac_Wilson_EvenOdd(0.5 / 0.12 - 4, u, ctx=c)
     src = ib.synth_point_sources(V // 2, 123)
-    slv = ib.Solver_CG(1e-20, 5000, ib.Fopr_DdagD(D), inner=inner)
+    slv = ib.Solver_CG(1e-20, 5000, ib.Fopr_DdagD(D), inner=inner, launched=launched)
     x, outs, rc = slv.solve_many(src.ravel(), 12)
     assert rc == ib.OK
     x = x.reshape(12, -1)
@@ -236,14 +242,15 @@ def test_multishift_stopped_mid_window_vs_oracle(port):
 
 # Lattices whose iterations run in one cooperative launch: fewer groups of 32
 # elements than SMs, one and several groups per block, a last group that is not
-# full (nrhs 3, 5: 10 and 6 sites a group), and the launched iteration just
-# above the rule's limit.
+# full (nrhs 3, 5: 10 and 6 sites a group), and lattices just above the rule's
+# limits for each storage (clover: 448, 1184 and 740 groups), which take the
+# launched iteration.
 @pytest.mark.parametrize("inner", ["double", "single", "half"])
 @pytest.mark.parametrize("op,L,nrhs", [
     ("wilson", [4, 4, 4, 8], 1), ("wilson", [8, 8, 8, 12], 1), ("wilson", [4, 6, 4, 4], 5),
     ("wilson_eo", [4, 4, 4, 8], 16), ("wilson_eo", [12, 12, 12, 16], 1), ("wilson_eo", [6, 4, 4, 6], 3),
     ("clover", [4, 4, 6, 4], 3), ("clover_eo", [2, 4, 4, 4], 12), ("clover_eo", [8, 8, 8, 16], 1),
-    ("clover_eo", [12, 12, 16, 16], 1)])
+    ("clover_eo", [12, 12, 16, 16], 1), ("clover_eo", [12, 16, 16, 16], 1), ("clover_eo", [16, 16, 16, 20], 1)])
 def test_cg_small_lattices(op, L, nrhs, inner):
     """The FP64 true residual of every solution, formed with the operators of
     the launched path (a different kernel), reaches the goal and is the one
@@ -265,6 +272,22 @@ def test_cg_small_lattices(op, L, nrhs, inner):
         res = np.linalg.norm(br - D.mult_dag(D.mult(xr))) / np.linalg.norm(br)
         assert res < 1.05 * TOL_RES and outs[r].diff < TOL_RES
         assert abs(res - outs[r].diff) < 1e-12 + 1e-2 * outs[r].diff
+
+
+def test_cg_small_lattice_over_several_launches():
+    """A launch of the one-launch iteration runs up to 256 iterations: a solve
+    near the critical mass takes more, and agrees with the launched iteration."""
+    L = [4, 4, 4, 8]
+    V = int(np.prod(L))
+    u = ib.synth_gauge(L, 0.2, 351, gauge_transform=True)
+    D = ib.Dirac_Wilson(0.5 / 0.128 - 4, u, ctx=ib.Context(L, 0))
+    b = ib.synth_gaussian(V, 352)
+    x, outs, rc = ib.Solver_CG(1e-20, 5000, ib.Fopr_DdagD(D)).solve_many(b, 1)
+    assert rc == ib.OK and outs[0].Iterations > 2 * 256 and outs[0].diff < TOL_RES
+    y, ref, rc = ib.Solver_CG(1e-20, 5000, ib.Fopr_DdagD(D), launched=True).solve_many(b, 1)
+    assert rc == ib.OK and abs(ref[0].Iterations - outs[0].Iterations) <= 0.05 * ref[0].Iterations
+    # both residuals are at 1e-10; the condition number of D^dag D is some 1e4
+    assert rel(x, y) < 1e4 * TOL_RES
 
 
 def test_cg_small_lattice_without_su3():
