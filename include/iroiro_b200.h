@@ -382,6 +382,12 @@ int iro_gcr_solve_field(iro_ctx* ctx, int op, double mass, double csw, const iro
    *waited_ms; the context stays usable. */
 int iro_selftest_bounded_wait(iro_ctx* ctx, double limit_ms, double* waited_ms);
 
+/* The same inside a solve: the barrier of the context's next small-lattice CG
+   finds one arrival missing and gives up after limit_ms (0 < limit_ms <= 1000).
+   That solve then starts again with launched iterations, as it does when the
+   barrier runs out by itself or the device refuses the cooperative launch. */
+int iro_selftest_cg_timeout(iro_ctx* ctx, double limit_ms);
+
 /* ---- synthetic inputs (host) ---------------------------------------------- */
 /* Seeded SU(3) field U = exp(i eps H), H = sum theta_a lambda_a / 2,
    theta_a ~ N(0,1), projected onto SU(3); optionally followed by a random

@@ -71,6 +71,7 @@ struct iro_ctx {
   unsigned* counter = nullptr;
   double* redout = nullptr;
   unsigned* sync_words = nullptr;  // the small-lattice CG's barrier counter and error flag
+  uint64_t cg_test_limit = 0;      // ns: the next small-lattice CG's barrier runs out (self-test)
   void* state = nullptr;  // CGState[16] or MSState
   int* done = nullptr;    // [16]
   void* h_pinned = nullptr;  // host mirror of state + done
@@ -1217,6 +1218,7 @@ GaugePtr gauge_small(iro_ctx* c, int prec) {
   return g;
 }
 unsigned* sync_words(iro_ctx* c) { return c->sync_words; }
+uint64_t& cg_test_limit(iro_ctx* c) { return c->cg_test_limit; }
 double* partials(iro_ctx* c) { return c->partials; }
 int sm_count(iro_ctx* c) { return c->sms; }
 bool gauge_loaded(iro_ctx* c) { return c->has_gauge; }

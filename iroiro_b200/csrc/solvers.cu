@@ -9,6 +9,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -53,6 +54,7 @@ int gauge_recon(iro_ctx* c);
 const double2* gauge_d18(iro_ctx* c);
 GaugePtr gauge_small(iro_ctx* c, int prec);
 unsigned* sync_words(iro_ctx* c);
+uint64_t& cg_test_limit(iro_ctx* c);
 double* partials(iro_ctx* c);
 int sm_count(iro_ctx* c);
 bool gauge_loaded(iro_ctx* c);
@@ -156,7 +158,11 @@ bool cg_is_small(int op, int prec, int nrhs, int64_t half_volume) {
 
 // Iterations from the device state until every right-hand side has left (or
 // paused): the inner loop of cg_double and cg_mixed on a small lattice.  A
-// launch is bounded to kSmallIters iterations (a few ms).
+// launch is bounded to kSmallIters iterations (a few ms).  kGaveUp when the
+// device refuses the cooperative launch or a wait at its barrier ran out (the
+// grid shares the device with work that holds it up): the fields are then
+// somewhere inside an iteration, and the solve starts again, launched.
+constexpr int kGaveUp = -1;
 constexpr int kSmallIters = 256;
 constexpr uint64_t kBarrierLimitNs = 1000000000ull;
 int iterate_small(iro_ctx* c, int op, double mass, const DevField* P, const DevField* Q, const DevField* R,
@@ -193,16 +199,25 @@ int iterate_small(iro_ctx* c, int op, double mass, const DevField* P, const DevF
   L.bar = sync_words(c);
   L.err = reinterpret_cast<int*>(sync_words(c) + 1);
   L.limit_ns = kBarrierLimitNs;
+  if (const uint64_t ns = std::exchange(cg_test_limit(c), 0)) {  // iro_selftest_cg_timeout
+    L.limit_ns = ns;
+    L.missing = 1;
+  }
   int* hpin = static_cast<int*>(pinned(c));
   for (int64_t launched = 0;;) {
-    CK(launch_cg_small(L, st));
+    const cudaError_t e = launch_cg_small(L, st);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+      cudaGetLastError();
+      return kGaveUp;
+    }
+    CK(e);
     launched += kSmallIters;
     CK(cudaMemcpyAsync(hpin, done(c), sizeof(int) * nrhs, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(hpin + 16, L.err, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (hpin[16]) {
       CK(cudaMemsetAsync(L.err, 0, sizeof(int), st));
-      return set_error(c, IRO_TIMEOUT, "a grid barrier of the small-lattice CG timed out");
+      return kGaveUp;
     }
     bool left = true;
     for (int r = 0; r < nrhs; ++r) left = left && hpin[r] != RUNNING;
@@ -214,8 +229,9 @@ bool want_graph(const iro_cg_params* prm) { return (prm->use_graph & ~IRO_CG_LAU
 bool want_launched(const iro_cg_params* prm) { return (prm->use_graph & IRO_CG_LAUNCHED) != 0; }
 
 // FP64 CG on D^dag D, Solver_CG::solve (lib/Solver/solver_CG.cpp:29-80).
+// launched: not in one cooperative launch, whatever the lattice
 int cg_double(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* prm,
-              const DevField* B, DevField* X, int nrhs, iro_solver_out* out) {
+              const DevField* B, DevField* X, int nrhs, iro_solver_out* out, bool launched) {
   const int sub = op_subset(op);
   const bool full = op_is_full(op);
   int rc = IRO_OK;
@@ -255,9 +271,11 @@ int cg_double(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* 
     return IRO_OK;
   };
   // (max_iter 0: no iteration, on either path)
-  if (prm->max_iter > 0 && !want_launched(prm) && cg_is_small(op, PREC_DOUBLE, nrhs, vh(c)))
-    RC(iterate_small(c, op, mass, P, Q, R, X, prm->max_iter));
-  else
+  if (prm->max_iter > 0 && !launched && cg_is_small(op, PREC_DOUBLE, nrhs, vh(c))) {
+    rc = iterate_small(c, op, mass, P, Q, R, X, prm->max_iter);
+    if (rc == kGaveUp) return cg_double(c, op, mass, csw, prm, B, X, nrhs, out, true);
+    RC(rc);
+  } else
     RC(iterate(c, nrhs, prm->max_iter, want_graph(prm), body));
   // true residual |A x - b| / |b| (solver_CG.cpp:69-71)
   RC(apply(c, op, mass, csw, false, *X, *Q, nullptr, 0, nullptr));
@@ -287,13 +305,15 @@ int cg_double(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* 
 // optional; the refinement of the mixed-precision multishift solve)
 int cg_mixed(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* prm,
              const DevField* B, DevField* X, int nrhs, iro_solver_out* out,
-             const double* sigma = nullptr, const double* target = nullptr);
+             const double* sigma = nullptr, const double* target = nullptr, bool launched = false);
 
 static int cg_any(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* prm,
                   const DevField* B, DevField* X, int nrhs, iro_solver_out* out) {
   auto t0 = std::chrono::steady_clock::now();
-  int rc = prm->inner_prec == PREC_DOUBLE ? cg_double(c, op, mass, csw, prm, B, X, nrhs, out)
-                                          : cg_mixed(c, op, mass, csw, prm, B, X, nrhs, out);
+  const bool launched = want_launched(prm);
+  int rc = prm->inner_prec == PREC_DOUBLE
+               ? cg_double(c, op, mass, csw, prm, B, X, nrhs, out, launched)
+               : cg_mixed(c, op, mass, csw, prm, B, X, nrhs, out, nullptr, nullptr, launched);
   auto t1 = std::chrono::steady_clock::now();
   const double ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
   for (int r = 0; r < nrhs; ++r) out[r].timing_ms = ms;
@@ -925,7 +945,7 @@ extern "C" int iro_rational_cg_solve(iro_ctx* c, int op, double mass, double csw
 // in Solver_CG (solver_CG.cpp:40).
 int cg_mixed(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* prm,
              const DevField* B, DevField* X, int nrhs, iro_solver_out* out, const double* sigma,
-             const double* target) {
+             const double* target, bool launched) {
   const int sub = op_subset(op);
   const bool full = op_is_full(op);
   const int pl = prm->inner_prec;
@@ -995,7 +1015,7 @@ int cg_mixed(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* p
     }
     return IRO_OK;
   };
-  const bool small = !shifted && !want_launched(prm) && cg_is_small(op, pl, nrhs, vh(c));
+  const bool small = !shifted && !launched && cg_is_small(op, pl, nrhs, vh(c));
   cudaGraphExec_t exec = nullptr;
   if (!small && want_graph(prm) && st != nullptr) {
     cudaGraph_t graph;
@@ -1017,7 +1037,11 @@ int cg_mixed(iro_ctx* c, int op, double mass, double csw, const iro_cg_params* p
   std::vector<int> hdone(nrhs), mask(nrhs);
   for (;;) {
     // inner iterations until some right-hand side pauses or all have left
-    if (small) RC(iterate_small(c, op, mass, Pl, Ql, Rl, Xl, prm->max_iter));
+    if (small) {
+      rc = iterate_small(c, op, mass, Pl, Ql, Rl, Xl, prm->max_iter);
+      if (rc == kGaveUp) return cg_mixed(c, op, mass, csw, prm, B, X, nrhs, out, sigma, target, true);
+      RC(rc);
+    }
     for (;;) {
       if (!small) {
         if (exec) CK(cudaGraphLaunch(exec, st));
@@ -1309,5 +1333,11 @@ extern "C" int iro_selftest_bounded_wait(iro_ctx* c, double limit_ms, double* wa
   CK(cudaStreamSynchronize(st));
   *waited_ms = double(hns) * 1e-6;
   if (herr) return set_error(c, IRO_TIMEOUT, "a grid barrier ran out (self-test)");
+  return IRO_OK;
+}
+
+extern "C" int iro_selftest_cg_timeout(iro_ctx* c, double limit_ms) {
+  if (!c || !(limit_ms > 0.0) || limit_ms > 1000.0) return IRO_BAD_ARG;
+  cg_test_limit(c) = uint64_t(limit_ms * 1e6);
   return IRO_OK;
 }
