@@ -293,8 +293,7 @@ HopLaunch base_launch(iro_ctx* c, int prec, bool dag, int nrhs) {
 // mixed-precision kernel on the FP16 links with three stored rows at 3, 4 or
 // 2 blocks per SM, any nrhs) and 13..14 (the same kernel on the 12-real FP16
 // links, row 2 rebuilt per link, at 3 or 4 blocks per SM); FP32 15 (24 warps
-// per SM, any nrhs).  IRO_HOP_VARIANT counts modulo the first 15.
-constexpr int kHopForced = 15;
+// per SM, any nrhs).
 constexpr int kHopVariants = 16;
 
 static bool variant_ok(const HopLaunch& L, int v) {
@@ -353,8 +352,8 @@ int launch_tuned(iro_ctx* c, HopLaunch L) {
     int v = 0, b = 256, g = 0;
     std::sscanf(forced, "%d,%d,%d", &v, &b, &g);
     if (L.prec == PREC_DOUBLE) v %= (L.recon == 12 ? 12 : 6);
-    else if (!variant_ok(L, v % kHopForced)) v %= 4;
-    else v %= kHopForced;
+    else if (!variant_ok(L, v % kHopVariants)) v %= 4;
+    else v %= kHopVariants;
     c->tuned[key] = Tune{v, b, g != 0};
     it = c->tuned.find(key);
   }
