@@ -289,7 +289,7 @@ HopLaunch base_launch(iro_ctx* c, int prec, bool dag, int nrhs) {
 // Candidates (see hop_var): all precisions 0..3; FP64 4, 5 and, on an SU(3)
 // field, 6..11 = 0..5 on the stored 18-real links (no third-row
 // reconstruction: fewer FP64 operations, more link bytes); FP32/FP16 with an
-// even nrhs 4..9 (two right-hand sides per thread); FP16 10..12 (the
+// even nrhs 4..7 (two right-hand sides per thread; 8 and 9 are not taken); FP16 10..12 (the
 // mixed-precision kernel on the FP16 links with three stored rows at 3, 4 or
 // 2 blocks per SM, any nrhs) and 13..14 (the same kernel on the 12-real FP16
 // links, row 2 rebuilt per link, at 3 or 4 blocks per SM); FP32 15 (24 warps
@@ -301,13 +301,13 @@ static bool variant_ok(const HopLaunch& L, int v) {
   if (v == 15) return L.prec == PREC_SINGLE;
   if (v < 4) return true;
   if (L.prec == PREC_DOUBLE) return v < 12 && (v < 6 || L.recon == 12);
-  if (v < 10) return L.recon == 12 && L.nrhs % 2 == 0;
+  if (v < 10) return v < 8 && L.recon == 12 && L.nrhs % 2 == 0;
   return L.prec == PREC_HALF && L.recon == 12;
 }
 
 // Candidates that are not timed: the FP64 variants of 128-thread blocks a second
 // time; the two-row links for full-lattice FP64 launches without clover blocks of
-// 8 right-hand sides and more; the staged kernels 8 and 9, which never won a shape.
+// 8 right-hand sides and more.
 // Rebuilding the third row per right-hand side won the tuner's few repeated
 // launches (two-row links of 12x20x28x44 about fit L2) and lost in a program's:
 // that lattice, variants 4 / 10, one field repeated and three in turn, 8
@@ -315,12 +315,10 @@ static bool variant_ok(const HopLaunch& L, int v) {
 // tie (283 / 278 us in turn), below that the bytes decide (1: 56 / 63 us); e/o
 // launches tie at 8 and 12 and keep both.
 static bool worth_timing(const HopLaunch& L, int v, int block) {
-  if (L.prec == PREC_DOUBLE) {
-    if (block > 128 && (v % 6 == 4 || v % 6 == 5)) return false;
-    const bool clov = L.epi == EPI_SCALE_CLOV || L.epi == EPI_XPAY_CLOV;
-    return !(L.recon == 12 && v < 6 && L.nparity == 2 && L.nrhs >= 8 && !clov);
-  }
-  return v != 8 && v != 9;
+  if (L.prec != PREC_DOUBLE) return true;
+  if (block > 128 && (v % 6 == 4 || v % 6 == 5)) return false;
+  const bool clov = L.epi == EPI_SCALE_CLOV || L.epi == EPI_XPAY_CLOV;
+  return !(L.recon == 12 && v < 6 && L.nparity == 2 && L.nrhs >= 8 && !clov);
 }
 
 static cudaError_t launch_variant(iro_ctx* c, HopLaunch L, cudaStream_t st) {

@@ -6,7 +6,6 @@
 
 #include "dslash.cuh"
 #include "dslash_pair.cuh"
-#include "dslash_stage.cuh"
 #include "internal.h"
 
 namespace iro {
@@ -117,56 +116,9 @@ static cudaError_t hop_go_pair(const HopLaunch& L, cudaStream_t st) {
   }
 }
 
-// two right-hand sides per thread with shared-memory staging of the neighbours
-template <int SP, int RECON, bool DAG, int EPI, int VAR>
-static cudaError_t hop_go_stage(const HopLaunch& L, cudaStream_t st) {
-  if constexpr (SP == PREC_DOUBLE || RECON != 12) {
-    return cudaErrorInvalidValue;
-  } else {
-    if (L.nrhs % 2 != 0 || L.hs0 != 0 || (L.nhs >= 0 && L.nhs != L.g.Vh)) return cudaErrorInvalidValue;
-    HopParams P;
-    P.g = L.g;
-    P.p0 = L.p0;
-    P.nrhs = L.nrhs;
-    for (int i = 0; i < 2; ++i) {
-      P.in[i] = L.in[i];
-      P.out[i] = L.out[i];
-      P.xin[i] = L.xin[i];
-      P.clov[i] = L.clov[i];
-    }
-    P.gauge = L.gauge;
-    P.scale = L.scale;
-    P.red_mask = L.red_mask;
-    P.red = L.red;
-    P.skip = L.skip;
-    P.cg = L.cg;
-    P.cst = L.cst;
-    for (int i = 0; i < 2; ++i) {
-      P.cr[i] = L.cr[i];
-    }
-    // the staging buffers of a block must fit the 227 KiB a block can opt in
-    // to (FP32: 976 B per thread, so at most 232 threads)
-    int cap = L.block_cap;
-    while (cap > 32 && stage_bytes<SP>() * cap > 232448) cap /= 2;
-    LaunchCfg c = launch_cfg(L.g.Vh, L.nrhs / 2, L.grid_cap(), cap);
-    if (stage_bytes<SP>() * c.block > 232448) return cudaErrorInvalidValue;
-    const int smem = stage_bytes<SP>() * c.block;
-    static int opted = 0;  // largest dynamic shared memory already allowed
-    if (smem > opted) {
-      cudaError_t e = cudaFuncSetAttribute(hop_stage_kernel<SP, DAG, EPI, VAR>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return e;
-      opted = smem;
-    }
-    dim3 grid(c.grid, L.nparity);
-    hop_stage_kernel<SP, DAG, EPI, VAR><<<grid, c.block, smem, st>>>(P);
-    return cudaGetLastError();
-  }
-}
-
 // Variants 0-3: hop_kernel (bits: see there).  FP32/FP16 with even nrhs:
 // 4-7 two right-hand sides per thread with the register cap none / 128 /
-// 152 / 168, 8-9 the same with the neighbours staged through shared memory.
+// 152 / 168.
 // FP64: 4/5 the 168-register 128-thread hop_kernel (5 with the rolled loop).
 // FP32, any nrhs: 15 the 80-register hop_kernel.
 // FP16 on links with three stored rows (RECON 18): only 10/11/12, the
@@ -211,8 +163,6 @@ static cudaError_t hop_var_more(const HopLaunch& L, cudaStream_t st) {
       case 5: return hop_go_pair<SP, RECON, DAG, EPI, 1>(L, st);
       case 6: return hop_go_pair<SP, RECON, DAG, EPI, 2>(L, st);
       case 7: return hop_go_pair<SP, RECON, DAG, EPI, 3>(L, st);
-      case 8: return hop_go_stage<SP, RECON, DAG, EPI, 0>(L, st);
-      case 9: return hop_go_stage<SP, RECON, DAG, EPI, 1>(L, st);
       default: break;
     }
     if constexpr (SP == PREC_SINGLE)
