@@ -307,13 +307,18 @@ static bool variant_ok(const HopLaunch& L, int v) {
 
 // Candidates that are not timed: the FP64 variants of 128-thread blocks a second
 // time; the two-row links for full-lattice FP64 launches without clover blocks of
-// 8 right-hand sides and more.
-// Rebuilding the third row per right-hand side won the tuner's few repeated
-// launches (two-row links of 12x20x28x44 about fit L2) and lost in a program's:
-// that lattice, variants 4 / 10, one field repeated and three in turn, 8
-// right-hand sides 370, 416 / 365, 361 us, 12 581, 658 / 556, 570 us.  At 6 they
-// tie (283 / 278 us in turn), below that the bytes decide (1: 56 / 63 us); e/o
-// launches tie at 8 and 12 and keep both.
+// 8 right-hand sides and more.  The third row is rebuilt per right-hand side, so
+// with many of them the stored row costs less; the tuner's few launches often
+// said otherwise.  Variants 4 / 10 and 0 / 6 on capped grids, sustained, us (one
+// context; two contexts whose launches overlap add up to 18 % to the two-row
+// ones):
+//   16^4        12 rhs  120 / 119, 131 / 132
+//   12x20x28x44  8 rhs  355 / 352, 352 / 352;  12 rhs  568 / 535, 587 / 590
+//   24^3x48      8 rhs  907 / 829, 809 / 815;  12 rhs 1354 / 1273, 1444 / 1447;  16 rhs 1793 / 1699, 1699 / 1710
+//   32^4        12 rhs 2155 / 2022, 2283 / 2309
+// (below 16^4 all are within 5 %).  At 6 right-hand sides the best of both tie,
+// below that the bytes decide (1, 12x20x28x44: 56 / 63 us); e/o launches tie at
+// 8 and 12 and keep both.
 static bool worth_timing(const HopLaunch& L, int v, int block) {
   if (L.prec != PREC_DOUBLE) return true;
   if (block > 128 && (v % 6 == 4 || v % 6 == 5)) return false;
