@@ -310,10 +310,6 @@ static bool variant_ok(const HopLaunch& L, int v) {
 // - FP32 15 below 6 right-hand sides, where variant 1 is the better one (e/o
 //   Wilson 16^3x32, 1 right-hand side 13.8 / 19.6 us, 5: 65 / 69; with another
 //   context's launches beside them 70 / 73 us on 22x20x32x44).
-// - Two FP64 blocks of 128 threads per SM where one of 256 fills it, in capped
-//   launches that sweep more than kSweepBytes: 128 / 256 threads, 24^3x48 clover,
-//   variant 0, 2 right-hand sides 279 / 284 us, 5: 906 / 836, and with another
-//   context's launches beside them 336 / 283 and 927 / 831.  Smaller sweeps tie.
 // - The two-row links for full-lattice FP64 launches without clover blocks of 8
 //   right-hand sides and more.  The third row is rebuilt per right-hand side, so
 //   with many of them the stored row costs less; the tuner's few launches often
@@ -326,14 +322,10 @@ static bool variant_ok(const HopLaunch& L, int v) {
 //   (below 16^4 all are within 5 %).  At 6 right-hand sides the best of both tie,
 //   below that the bytes decide (1, 12x20x28x44: 56 / 63 us); e/o launches tie
 //   at 8 and 12 and keep both.
-constexpr int64_t kSweepBytes = int64_t(200) << 20;
-static bool worth_timing(const HopLaunch& L, int v, int block, bool free_grid) {
+static bool worth_timing(const HopLaunch& L, int v, int block) {
   if (L.prec == PREC_SINGLE) return v != 15 || L.nrhs >= 6;
   if (L.prec != PREC_DOUBLE) return true;
-  const bool small_regs = v % 6 == 4 || v % 6 == 5;  // 128-thread blocks only
-  if (block > 128 && small_regs) return false;
-  const int64_t sweep = int64_t(L.nparity) * L.g.Vh * L.nrhs * 192;
-  if (block <= 128 && !small_regs && !free_grid && sweep > kSweepBytes) return false;
+  if (block > 128 && (v % 6 == 4 || v % 6 == 5)) return false;
   const bool clov = L.epi == EPI_SCALE_CLOV || L.epi == EPI_XPAY_CLOV;
   return !(L.recon == 12 && v < 6 && L.nparity == 2 && L.nrhs >= 8 && !clov);
 }
@@ -392,7 +384,7 @@ int launch_tuned(iro_ctx* c, HopLaunch L) {
     for (int v = 0; v < kHopVariants; ++v)
       for (int b : {256, 128})
         for (int g : {0, 1}) {
-          if (!variant_ok(L, v) || !worth_timing(L, v, b, g != 0)) continue;
+          if (!variant_ok(L, v) || !worth_timing(L, v, b)) continue;
           T.variant = v;
           T.block_cap = b;
           T.grid_free = g;

@@ -184,10 +184,12 @@ struct HopBounds {
   static constexpr int blocks =
       (VAR & 16) ? 3 : (VAR & 8) ? ((VAR & 1) ? 4 : ((VAR & 2) ? 2 : 3))
                 : ((VAR & 4) ? 3 : ((VAR & 1) ? 2 : 1));
+  // the blocks of an SM as one (resident_grid): the same register cap
+  static constexpr int full = threads * blocks;
 };
 
 template <int SP, int GP, int RECON, bool DAG, int EPI, int CP, int VAR>
-__global__ void __launch_bounds__(HopBounds<VAR>::threads, HopBounds<VAR>::blocks)
+__global__ void __launch_bounds__(HopBounds<VAR>::full, 1)
     hop_kernel(HopParams P) {
   using R = typename SpinorIO<SP>::Real;
   // Launched as a programmatic dependent launch (hop_go): wait until the

@@ -35,6 +35,24 @@ static int resident_grid(const LaunchCfg& c, const HopLaunch& L) {
   return c.grid > fit ? (fit > 0 ? fit : 1) : c.grid;
 }
 
+// The same as one block per SM.  Blocks of another stream's launch take an SM's
+// slots one by one as this launch's blocks leave them; with several per SM the
+// two launches then run half and half through all of their length, and from
+// kSweepBytes of spinors on the slices that neighbours share no longer fit L2
+// for both.  Applications, us, one context / contexts in turn, small blocks and
+// one per SM: FP32 clover 28x20x26x66, 16 right-hand sides, 1520 / 1763, 1482 /
+// 1703; FP64 clover 32x26x30x34, 2: 364 / 429, 359 / 359; FP16 e/o 32^3x64, 5:
+// 596 / 633, 580 / 587.  Launches that reduce keep the small blocks
+// (block_reduce_finish takes 256 threads).
+constexpr int64_t kSweepBytes = int64_t(200) << 20;
+static void block_per_sm(LaunchCfg& c, const HopLaunch& L, int full, int nthreads) {
+  if (L.red_mask || L.cg || full <= c.block || int64_t(c.grid) * c.block >= nthreads) return;
+  const int site = L.prec == PREC_DOUBLE ? 192 : L.prec == PREC_SINGLE ? 96 : 52;
+  if (int64_t(L.nparity) * L.g.Vh * L.nrhs * site < kSweepBytes) return;
+  c.block = full / L.nrhs * L.nrhs;
+  c.grid = L.max_blocks / 8 / L.nparity;
+}
+
 template <int SP, int GP, int RECON, bool DAG, int EPI, int VAR>
 static cudaError_t hop_go(const HopLaunch& L, cudaStream_t st) {
   HopParams P;
@@ -64,6 +82,7 @@ static cudaError_t hop_go(const HopLaunch& L, cudaStream_t st) {
                            L.block_cap < HopBounds<VAR>::threads ? L.block_cap
                                                                  : HopBounds<VAR>::threads);
   c.grid = resident_grid<hop_kernel<SP, GP, RECON, DAG, EPI, SP, VAR>>(c, L);
+  block_per_sm(c, L, HopBounds<VAR>::full, P.nhs * L.nrhs);
   // programmatic dependent launch: the blocks of this grid may be scheduled
   // while the previous kernel's last blocks retire (hop_kernel waits for
   // that kernel's completion before it reads anything), hiding the launch

@@ -119,3 +119,28 @@ def test_capped_grids_and_divisions(op, nrhs):
     if op == "OP_WILSON_FULL" and nrhs >= 8:
         picked = [t["variant"] for t in c.autotune_report() if t["prec"] == 0 and t["nrhs"] == nrhs]
         assert picked and min(picked) >= 6  # the three-row links
+
+
+@pytest.mark.parametrize("op,nrhs", [("OP_WILSON_FULL", 5), ("OP_WILSON_FULL", 16), ("OP_CLOVER_FULL", 12),
+                                     ("OP_WILSON_HOP_EO", 16)])
+def test_one_block_per_sm(op, nrhs):
+    """Launches that sweep more than 200 MiB of spinors run as one block per SM,
+    of as many threads as its registers let in (rounded down to a multiple of
+    the right-hand sides: 380 of 384 for 5).  The right-hand sides are one field
+    times 2^r, so that each must be 2^r times the one-right-hand-side result."""
+    import numpy as np
+
+    import iroiro_b200 as ib
+    L, code = [24, 24, 24, 32], getattr(ib, op)
+    n = int(np.prod(L)) // (2 if "HOP" in op else 1)
+    c = ib.Context(L, 0)
+    c.upload_gauge(ib.synth_gauge(L, 0.2, 431), force=True)
+    m, csw = 0.5 / 0.12 - 4, 1.0
+    f = ib.synth_gaussian(n, 432)
+    ref = c.apply(code, m, csw, 1, f, "double")
+    norm = np.linalg.norm(ref)
+    many = np.concatenate([np.ldexp(f, r) for r in range(nrhs)])
+    for prec, tol in (("double", 150 * 1.1e-16), ("single", TOL_FP32), ("half", TOL_FP16)):
+        got = c.apply(code, m, csw, 1, many, prec, nrhs=nrhs).reshape(nrhs, -1)
+        for r in range(nrhs):
+            assert np.linalg.norm(np.ldexp(got[r], -r) - ref) < tol * norm, (prec, r)
