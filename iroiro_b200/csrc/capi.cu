@@ -387,6 +387,7 @@ int launch_tuned(iro_ctx* c, HopLaunch L) {
           if (!variant_ok(L, v) || !worth_timing(L, v, b)) continue;
           T.variant = v;
           T.block_cap = b;
+          T.tuning = 1;
           T.grid_free = g;
           CK(launch_variant(c, T, st));  // warm-up
           CK(cudaEventRecord(e0, st));

@@ -43,10 +43,13 @@ static int resident_grid(const LaunchCfg& c, const HopLaunch& L) {
 // one per SM: FP32 clover 28x20x26x66, 16 right-hand sides, 1520 / 1763, 1482 /
 // 1703; FP64 clover 32x26x30x34, 2: 364 / 429, 359 / 359; FP16 e/o 32^3x64, 5:
 // 596 / 633, 580 / 587.  Launches that reduce keep the small blocks
-// (block_reduce_finish takes 256 threads).
+// (block_reduce_finish takes 256 threads), and a shape's variant is tuned with
+// them: one block per SM levels the variants (FP16 e/o 32^3x64, 12 right-hand
+// sides, variants 10 / 12: 1345 / 1346 us, small blocks 1370 / 1540), and 12
+// picked on that made the solve with its reductions 5 % slower.
 constexpr int64_t kSweepBytes = int64_t(200) << 20;
 static void block_per_sm(LaunchCfg& c, const HopLaunch& L, int full, int nthreads) {
-  if (L.red_mask || L.cg || full <= c.block || int64_t(c.grid) * c.block >= nthreads) return;
+  if (L.red_mask || L.cg || L.tuning || full <= c.block || int64_t(c.grid) * c.block >= nthreads) return;
   const int site = L.prec == PREC_DOUBLE ? 192 : L.prec == PREC_SINGLE ? 96 : 52;
   if (int64_t(L.nparity) * L.g.Vh * L.nrhs * site < kSweepBytes) return;
   c.block = full / L.nrhs * L.nrhs;

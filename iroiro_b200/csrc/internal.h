@@ -55,6 +55,7 @@ struct HopLaunch {
   int max_blocks;
   int variant;    // kernel variant (see hop_kernel), chosen by the autotuner
   int block_cap;  // largest block size (128 or 256), chosen by the autotuner
+  int tuning = 0;  // a timing launch of the autotuner: blocks as in a launch that reduces
   // fused CG update on the output (see HopParams::cg)
   int cg = 0;
   SpinorPtr cr[2];
