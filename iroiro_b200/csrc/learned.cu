@@ -176,13 +176,15 @@ __device__ __forceinline__ void mma_16816(float c[4], const uint32_t a[4], uint3
 //
 // The sum of a tile (96 rows) is FP32 with FMAs; tiles are added in FP64, in
 // the CTA's own block of `partial`, in the order of the tiles, and the CTAs in
-// block order.  The tensor cores take the same products at a quarter of the
-// time, but truncate their FP32 sums: their error was one-sided and grew with
+// block order.  The tensor cores take the same products faster (a 16->16 layer
+// at 16^3x32 147 us, 277 us here; a training step of (4,16,16,16,4) 1.19 and
+// 1.51 ms), but truncate their FP32 sums: the error was one-sided and grew with
 // the volume, on unit links against a 64-bit sum of the same operands 2.6e-7 at
-// 8^3x16, 3.4e-6 at 16^3x32, 1.7e-5 at 24^3x48, against 3.3e-8 (the result's own rounding) here at all three.
+// 8^3x16, 3.4e-6 at 16^3x32, 1.7e-5 at 24^3x48, where it is 3.3e-8 here, the
+// rounding of the result.
 //
-// Bound by the FMAs and their operand loads.  A training step of
-// (4,16,16,16,4) at 16^3x32 takes 1.51 ms with it, 1.19 ms on the tensor cores.
+// Bound by the operand loads from shared memory (L1 busy 78 %) and the FMAs.
+// Blocks of 4 x 8 with BF16 rows of A, half the loads, took the same time.
 template <int CIN, int COUT>
 struct PtcDb {
   static constexpr int NF = 2 * COUT;
@@ -382,9 +384,6 @@ struct PtcLayer {
   static constexpr int RED_BYTES = 4 * 6 * NT * 32 * 16;
 };
 
-// The channels of displacement D at one site, transported, as BF16 rows of the
-// warp's staging tile: row 32 colour + lane holds the real parts of the
-// channels, then the imaginary parts.  Then their product with the weights.
 // The feature rows and links of the next direction, requested into L1 while the
 // present one is multiplied: the loads of a direction wait ~7 issue slots per
 // instruction on L2 otherwise (long scoreboard; 20 warps an SM).
@@ -469,6 +468,9 @@ __device__ __forceinline__ void mul_dir4(const RawDir& r, int D, const uint32_t*
   }
 }
 
+// The channels of displacement D at one site, transported, as BF16 rows of the
+// warp's staging tile: row 32 colour + lane holds the real parts of the
+// channels, then the imaginary parts.  Then their product with the weights.
 // KIND 0: the site itself; 1: forward, 2: backward along mu (a run-time index:
 // one copy of the code per kind, and no direction's loads hoisted over
 // another's, which spilled)
